@@ -19,6 +19,7 @@
 #include "kernels.h"
 #include "kernels_flatten.h"
 #include "fill.h"
+#include "stroke_verbs.h"
 
 namespace {
 
@@ -58,6 +59,16 @@ struct lyon_gpu_context {
     bool order_valid = false;
     DevBuf path_class, class_counters;  // classification for the one-thread-per-path phase
     bool split_valid = false;           // class_counters holds the first short item
+    // the verb-parallel stroke (stroke_verbs.cu): its arrays per verb and per path
+    DevBuf verb_mem, verb_paths;
+    lg::SideStreams side;       // made with the first such call, of the stream's priority
+    bool side_made = false;
+    uint32_t verb_cap = 0;      // verbs verb_mem holds
+    uint32_t verb_count = 0;    // verbs of the last counted batch
+    uint32_t verbs_known = 0;   // the coming batch's verbs when the caller knows them, else 0
+    bool verbs_valid = false;   // the last count phase was verb-parallel
+    bool verb_runs = false;     // its batch has curves with interior steps
+    uint32_t walk_paths = 0;    // its paths left to the walk
     // stroke launch settings (the autotuner's knobs)
     uint32_t long_path_points = 1024;  // paths with more points go first; 0: path order
     uint32_t blocks_per_sm = 0;        // 0: as many as fit
@@ -248,11 +259,25 @@ bool alloc_path_arrays(lyon_gpu_context* ctx, uint32_t n) {
 
 // Index-range policy + scan + totals. On return the offsets are valid and *tv / *ti hold the
 // totals (one host synchronisation).
+// With `verbs`, the counts come from the verb-parallel stroke: its words are read with the totals,
+// and the paths it left are walked before the second pass. Returns with verbs->retry set, and no
+// totals, when the batch has to be counted again (more verbs than the arrays hold, or offsets it
+// cannot work from).
+struct VerbCount {
+    const lg::StrokeArgs* args;
+    const lg::StrokeVerbs* arrays;
+    int grid;
+    uint32_t words[lg::STROKE_VERBS_READ];
+    bool retry;
+};
 bool finish_counts(lyon_gpu_context* ctx, uint32_t n, int index_bits, int index_mode,
-                   uint64_t vertex_offset, uint64_t* tv, uint64_t* ti, uint32_t* failed) {
+                   uint64_t vertex_offset, uint64_t* tv, uint64_t* ti, uint32_t* failed,
+                   VerbCount* verbs = nullptr) {
     cudaStream_t s = ctx->stream;
     uint32_t* sw = small_words(ctx);
     uint64_t maxi = max_index_for(index_bits);
+    bool to_walk = verbs != nullptr;
+again:
     cudaMemsetAsync(sw + 2, 0, 8, s);
     // Per-path mode applies the index range per path; the global mode only counts failures.
     if (!set_err(ctx, "per-path limit",
@@ -275,8 +300,12 @@ bool finish_counts(lyon_gpu_context* ctx, uint32_t n, int index_bits, int index_
         uint64_t* hs_dev = direct_host_pointer<uint64_t>(hs);
         if (hs_dev) {
             lg::launch_read_totals(as<uint64_t>(ctx->vtx_offsets) + n,
-                                   as<uint64_t>(ctx->idx_offsets) + n, sw + 2, hs_dev, s);
+                                   as<uint64_t>(ctx->idx_offsets) + n, sw + 2,
+                                   verbs ? verbs->arrays->words : nullptr, hs_dev, s);
         } else {
+            if (verbs)
+                cudaMemcpyAsync(hs + 3, verbs->arrays->words, sizeof verbs->words,
+                                cudaMemcpyDeviceToHost, s);
             cudaMemcpyAsync(hs, as<uint64_t>(ctx->vtx_offsets) + n, 8, cudaMemcpyDeviceToHost, s);
             cudaMemcpyAsync(hs + 1, as<uint64_t>(ctx->idx_offsets) + n, 8, cudaMemcpyDeviceToHost,
                             s);
@@ -291,6 +320,24 @@ bool finish_counts(lyon_gpu_context* ctx, uint32_t n, int index_bits, int index_
             return false;
         }
         *failed = hw[1];
+        if (to_walk) {
+            to_walk = false;
+            memcpy(verbs->words, hs + 3, sizeof verbs->words);
+            if (verbs->words[0] > verbs->arrays->cap || verbs->words[1] != 0) {
+                verbs->retry = true;
+                return true;
+            }
+            if (verbs->words[2] > 0) {
+                lg::StrokeArgs w = *verbs->args;
+                w.order = verbs->arrays->walk_list;
+                w.item_split = verbs->arrays->words + 2;
+                w.list_only = 1;
+                cudaMemsetAsync(w.work_counter, 0, 4, s);
+                if (!set_err(ctx, "stroke count", lg::launch_stroke(w, false, verbs->grid, s)))
+                    return false;
+                goto again;
+            }
+        }
         if (index_mode == LYON_INDEX_GLOBAL && *tv > 0 && vertex_offset + *tv - 1 > maxi &&
             pass == 0) {
             if (!global_overflow_fixup(ctx, n, vertex_offset, maxi)) return false;
@@ -363,6 +410,121 @@ int stroke_grid(lyon_gpu_context* ctx, uint32_t n) {
     return needed < max_grid ? (needed > 0 ? needed : 1) : max_grid;
 }
 
+// The verb-parallel stroke's arrays, cut from one allocation.
+lg::StrokeVerbs stroke_verbs(lyon_gpu_context* ctx, uint32_t n) {
+    lg::StrokeVerbs v;
+    const size_t cap = ctx->verb_cap;
+    unsigned char* m = as<unsigned char>(ctx->verb_mem);
+    auto take = [&](size_t bytes) {
+        unsigned char* p = m;
+        m += bytes;
+        return p;
+    };
+    v.words = reinterpret_cast<uint32_t*>(take(lg::STROKE_VERBS_WORDS * 4));
+    v.scan = reinterpret_cast<unsigned long long*>(take(2 * lg::scan_tile_count(ctx->verb_cap) * 8));
+    v.clear_bytes = (size_t)(m - as<unsigned char>(ctx->verb_mem));
+    v.cap = ctx->verb_cap - 1;
+    v.firsts = reinterpret_cast<float4*>(take(cap * 16));
+    v.lasts = reinterpret_cast<float4*>(take(cap * 16));
+    v.fin = reinterpret_cast<float2*>(take(cap * 8));
+    v.rec = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.path = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.join = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.split = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.drops = v.split;
+    v.cut = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.extra = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.irregular = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.vpre = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.ipre = reinterpret_cast<uint32_t*>(take(cap * 4));
+    v.flags = reinterpret_cast<uint16_t*>(take(cap * 2));
+    v.kind = take(cap);
+    v.path_walk = as<uint32_t>(ctx->verb_paths);
+    v.walk_list = v.path_walk + n;
+    v.path_v = v.walk_list + n;
+    v.path_i = v.path_v + n;
+    return v;
+}
+
+// Room for `verbs` verbs (whole scan tiles, so that every array starts on a 16-byte boundary).
+bool grow_verbs(lyon_gpu_context* ctx, uint32_t verbs) {
+    if (verbs < ctx->verb_cap) return true;
+    const uint64_t cap = ((uint64_t)verbs + verbs / 8 + 2048) / 2048 * 2048;
+    if (cap > 0xFFFFF000ull) return false;
+    ctx->verb_cap = 0;
+    if (!ensure(ctx, ctx->verb_mem, cap * lg::STROKE_VERBS_BYTES + lg::STROKE_VERBS_WORDS * 4 +
+                                        2 * lg::scan_tile_count((uint32_t)cap) * 8))
+        return false;
+    ctx->verb_cap = (uint32_t)cap;
+    return true;
+}
+
+const lg::SideStreams& side_streams(lyon_gpu_context* ctx) {
+    if (!ctx->side_made) {
+        ctx->side_made = true;
+        int priority = 0;
+        cudaStreamGetPriority(ctx->stream, &priority);
+        for (int i = 0; i < 2; ++i) {
+            lg::SideStreams& d = ctx->side;
+            if (cudaStreamCreateWithPriority(&d.stream[i], cudaStreamNonBlocking, priority) !=
+                    cudaSuccess ||
+                cudaEventCreateWithFlags(&d.forked[i], cudaEventDisableTiming) != cudaSuccess ||
+                cudaEventCreateWithFlags(&d.joined[i], cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                if (d.stream[i]) cudaStreamDestroy(d.stream[i]);
+                d.stream[i] = nullptr;
+            }
+        }
+    }
+    return ctx->side;
+}
+
+// Counts a fixed-width stroke of positions verb by verb. Returns LYON_OK with ctx->verbs_valid
+// false when the batch is left to the path-by-path count (its offsets overlap, or no room for the
+// arrays).
+int count_by_verb(lyon_gpu_context* ctx, const lyon_path_batch* batch,
+                  const lyon_stroke_options* options, uint32_t num_options, int index_bits,
+                  int index_mode, uint64_t vertex_offset, uint64_t* tv, uint64_t* ti,
+                  uint32_t* failed) {
+    const uint32_t n = batch->num_paths;
+    cudaStream_t s = ctx->stream;
+    uint32_t need = ctx->verbs_known;
+    if (need == 0 && ctx->verb_cap == 0) {
+        // The first batch: its size is on the device. Later ones are tried with the arrays there
+        // are, and counted again when they hold more.
+        uint32_t ends[2] = {0, 0};
+        cudaMemcpyAsync(&ends[0], batch->verb_offsets, 4, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(&ends[1], batch->verb_offsets + n, 4, cudaMemcpyDeviceToHost, s);
+        if (!set_err(ctx, "sync", cudaStreamSynchronize(s))) return LYON_ERR_CUDA;
+        need = ends[1] > ends[0] ? ends[1] - ends[0] : 1u;
+    }
+    if (!ensure(ctx, ctx->verb_paths, (size_t)n * 16)) return LYON_OK;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        if (!grow_verbs(ctx, need)) return LYON_OK;
+        const lg::StrokeVerbs v = stroke_verbs(ctx, n);
+        const lg::StrokeArgs a = stroke_args(ctx, batch, options, num_options, index_bits,
+                                             index_mode, vertex_offset);
+        const uint32_t hint = need ? need : ctx->verb_count > n ? ctx->verb_count : n;
+        if (!set_err(ctx, "stroke count",
+                     lg::launch_stroke_verbs_count(a, v, hint, ctx->num_sms, side_streams(ctx), s)))
+            return LYON_ERR_CUDA;
+        VerbCount c{&a, &v, stroke_grid(ctx, n), {}, false};
+        mark(ctx, 1);
+        if (!finish_counts(ctx, n, index_bits, index_mode, vertex_offset, tv, ti, failed, &c))
+            return LYON_ERR_CUDA;
+        if (!c.retry) {
+            ctx->verb_count = c.words[0];
+            ctx->walk_paths = c.words[2];
+            ctx->verb_runs = c.words[3] != 0;
+            ctx->verbs_valid = true;
+            return LYON_OK;
+        }
+        if (c.words[1] != 0) return LYON_OK;
+        need = c.words[0];
+    }
+    return LYON_OK;
+}
+
 // Count pass + scan for one device-resident batch.
 int pipeline_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch,
                    const void* options, uint32_t num_options, int index_bits, int index_mode,
@@ -373,6 +535,17 @@ int pipeline_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch
     mark(ctx, 0);
     ctx->order_valid = false;
     ctx->split_valid = false;
+    ctx->verbs_valid = false;
+    if (kind == KIND_STROKE && n > 0 && !ctx->vw_widths && !ctx->want_sources &&
+        !ctx->vertex_attrs) {
+        const int r = count_by_verb(ctx, batch, (const lyon_stroke_options*)options, num_options,
+                                    index_bits, index_mode, vertex_offset, tv, ti, failed);
+        if (r != LYON_OK) return r;
+        if (ctx->verbs_valid) {
+            mark(ctx, 2);
+            return LYON_OK;
+        }
+    }
     if (kind == KIND_STROKE) {
         // Long paths first, so that no single long path is left running at the end of a launch;
         // short line-only paths last, for the one-thread-per-path phase.
@@ -432,7 +605,22 @@ int pipeline_emit(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch,
                                        num_options, index_bits, index_mode, vertex_offset);
         a.vertices = vout;
         a.indices = iout;
-        if (n > 0 && tv > 0) {
+        if (n > 0 && tv > 0 && ctx->verbs_valid) {
+            const lg::StrokeVerbs v = stroke_verbs(ctx, n);
+            if (!set_err(ctx, "stroke emit",
+                         lg::launch_stroke_verbs_emit(a, v, ctx->verb_count, ctx->verb_runs,
+                                                      ctx->num_sms, side_streams(ctx), s)))
+                return LYON_ERR_CUDA;
+            if (ctx->walk_paths > 0) {
+                a.order = v.walk_list;
+                a.item_split = v.words + 2;
+                a.list_only = 1;
+                cudaMemsetAsync(small_words(ctx), 0, 4, s);
+                if (!set_err(ctx, "stroke emit",
+                             lg::launch_stroke(a, true, stroke_grid(ctx, ctx->walk_paths), s)))
+                    return LYON_ERR_CUDA;
+            }
+        } else if (n > 0 && tv > 0) {
             cudaMemsetAsync(small_words(ctx), 0, 4, s);
             if (a.seq_counter) cudaMemsetAsync(a.seq_counter, 0, 4, s);
             if (!set_err(ctx, "stroke emit", lg::launch_stroke(a, true, stroke_grid(ctx, n), s)))
@@ -618,8 +806,10 @@ int batched_host(lyon_gpu_context* ctx, int kind, const lyon_path_batch* hb, con
         uint64_t tv = 0, ti = 0;
         uint32_t failed = 0;
         uint64_t voff = index_mode == LYON_INDEX_GLOBAL ? vertex_offset + run_v : vertex_offset;
+        ctx->verbs_known = ve - vb;
         int r = pipeline_count(ctx, kind, &db, ctx->h_in_opts.ptr, num_options > 1 ? cn : 1,
                                index_bits, index_mode, voff, &tv, &ti, &failed);
+        ctx->verbs_known = 0;
         if (r != LYON_OK) return r;
         if (run_v + tv > vcap || run_i + ti > icap || !hv || (ti && !hi)) capacity_ok = false;
         if (capacity_ok && cn > 0) {
@@ -734,8 +924,10 @@ int single_path(lyon_gpu_context* ctx, int kind, const uint8_t* verbs, uint32_t 
         ctx->width_stride = floats_per_point;
     }
     lyon_gpu_batch_output bo;
+    ctx->verbs_known = num_verbs;
     int r = batched_device(ctx, kind, &b, ctx->in_options.ptr, 1, index_bits,
                            LYON_INDEX_PER_PATH, index_base, &bo);
+    ctx->verbs_known = 0;
     if (r != LYON_OK) return r;
     cudaStream_t s = ctx->stream;
     if (!ensure_host(ctx, ctx->h_small, 64)) return LYON_ERR_OUT_OF_MEMORY;
@@ -798,13 +990,15 @@ int single_path(lyon_gpu_context* ctx, int kind, const uint8_t* verbs, uint32_t 
 namespace lg {
 
 int srv_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch, const void* options,
-              uint32_t num_options, const uint32_t* request_first, uint64_t* tv, uint64_t* ti,
-              uint32_t* failed) {
+              uint32_t num_options, uint32_t num_verbs, const uint32_t* request_first,
+              uint64_t* tv, uint64_t* ti, uint32_t* failed) {
     cudaSetDevice(ctx->device);
+    ctx->verbs_known = num_verbs;
     ctx->request_first = request_first;
     int r = pipeline_count(ctx, kind, batch, options, num_options, 32, LYON_INDEX_GLOBAL, 0, tv,
                            ti, failed);
     ctx->request_first = nullptr;
+    ctx->verbs_known = 0;
     return r;
 }
 
@@ -969,7 +1163,7 @@ void lyon_gpu_destroy(lyon_gpu_context* ctx) {
                       &ctx->hatch_bound,
                       &ctx->hatch_edge_count, &ctx->hatch_counts, &ctx->hatch_status,
                       &ctx->hatch_offsets, &ctx->hatch_scratch, &ctx->hatch_out,
-                      &ctx->hatch_order};
+                      &ctx->hatch_order, &ctx->verb_mem, &ctx->verb_paths};
     for (DevBuf* b : bufs) free_buf(*b);
     lg::fill_free(ctx->fill);
     HostBuf* hb[] = {&ctx->h_verbs, &ctx->h_points, &ctx->h_out_v,  &ctx->h_out_i,
@@ -981,6 +1175,11 @@ void lyon_gpu_destroy(lyon_gpu_context* ctx) {
     for (int i = 0; i < 2; ++i)
         if (ctx->slot_done[i]) cudaEventDestroy(ctx->slot_done[i]);
     if (ctx->emitted) cudaEventDestroy(ctx->emitted);
+    for (int i = 0; i < 2; ++i) {
+        if (ctx->side.forked[i]) cudaEventDestroy(ctx->side.forked[i]);
+        if (ctx->side.joined[i]) cudaEventDestroy(ctx->side.joined[i]);
+        if (ctx->side.stream[i]) cudaStreamDestroy(ctx->side.stream[i]);
+    }
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;

@@ -89,14 +89,13 @@ __host__ __device__ __forceinline__ uint32_t to_u32_or1(float n) {
 
 // ---- flattening segment counts (quadratic_bezier.rs:943-974, cubic_bezier.rs:1369-1403) -----
 __host__ __device__ __forceinline__ float wang_from_err4(float err4) {
-    // i^4 for i in 1..=24; the first i with err4 <= i^4 is ceil(err4^(1/4)).
+    // The first i in 1..=24 with err4 <= i^4 is ceil(err4^(1/4)): two rounded square roots come
+    // within one of it, and the comparison with i^4 (exact in f32) settles which.
     if (err4 <= 331776.0f) {
-#pragma unroll 1
-        for (int i = 1; i <= 24; ++i) {
-            float f = (float)i;
-            float lut = (f * f) * (f * f);
-            if (err4 <= lut) return f;
-        }
+        const float i = fmaxf(ceilf(sqrtf(sqrtf(err4))), 1.0f);
+        const float h = i - 1.0f;
+        if (err4 > (i * i) * (i * i)) return i + 1.0f;
+        return h >= 1.0f && err4 <= (h * h) * (h * h) ? h : i;
     }
     return fmaxf(sqrtf(sqrtf(err4)), 1.0f);
 }

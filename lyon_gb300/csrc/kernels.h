@@ -48,6 +48,8 @@ struct StrokeArgs {
     // warp items left; `seq_counter` (zeroed before each launch) hands out those.
     const uint32_t* item_split;
     uint32_t* seq_counter;
+    // Non-zero: only items [0, *item_split) of the order are stroked.
+    int list_only;
     // Non-zero: every path is stroked by lyon's sequential stepper, one path per thread, in both
     // passes (set by the custom-attribute calls; `widths` implies it). With `sources` the emit
     // pass writes each vertex's lyon_vertex_source next to it.
@@ -162,8 +164,10 @@ cudaError_t launch_svg_parse(const char* text, const uint64_t* string_offsets, u
 // Writes out_a[n], out_b[n] (the scan totals) and the two u32 words at `words` into `host_dst`
 // (mapped pinned host memory) with a kernel, so that the read-back does not queue behind large
 // device->host copies on the copy engines.
+// With `more`, four more words follow.
 cudaError_t launch_read_totals(const uint64_t* a_total, const uint64_t* b_total,
-                               const uint32_t* words, uint64_t* host_dst, cudaStream_t s);
+                               const uint32_t* words, const uint32_t* more, uint64_t* host_dst,
+                               cudaStream_t s);
 
 // Processing order by class: paths with more than `big_points` points (0: none) first, then the
 // other paths, then line-only paths of at most `short_points` points (0: none; at most

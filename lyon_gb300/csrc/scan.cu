@@ -9,6 +9,7 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "scan_core.cuh"
 
 namespace lg {
 
@@ -16,67 +17,7 @@ static std::atomic<uint64_t> g_launches{0};
 void note_launches(uint32_t k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
 uint64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
 
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-constexpr unsigned long long FLAG_AGG = 1ull << 62;
-constexpr unsigned long long FLAG_INC = 2ull << 62;
-constexpr unsigned long long VALUE_MASK = (1ull << 62) - 1;
-constexpr uint32_t SPIN_LIMIT = 1u << 24;
-
 __host__ __device__ size_t scan_tile_count(uint32_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
-
-__device__ __forceinline__ unsigned long long block_excl_scan(unsigned long long v,
-                                                              unsigned long long* total) {
-    __shared__ unsigned long long warp_sums[SCAN_THREADS / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned long long x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long n = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += n;
-    }
-    if (lane == 31) warp_sums[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        unsigned long long s = lane < SCAN_THREADS / 32 ? warp_sums[lane] : 0ull;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long n = __shfl_up_sync(0xFFFFFFFFu, s, o);
-            if (lane >= o) s += n;
-        }
-        if (lane < SCAN_THREADS / 32) warp_sums[lane] = s;
-    }
-    __syncthreads();
-    unsigned long long before = w > 0 ? warp_sums[w - 1] : 0ull;
-    *total = warp_sums[SCAN_THREADS / 32 - 1];
-    __syncthreads();
-    return before + x - v;
-}
-
-// Looks back from `tile` and returns the exclusive prefix of one channel.
-__device__ __forceinline__ unsigned long long look_back(unsigned long long* state, uint32_t tile,
-                                                        int* error) {
-    unsigned long long prefix = 0;
-    int64_t j = (int64_t)tile - 1;
-    while (j >= 0) {
-        unsigned long long s;
-        uint32_t spins = 0;
-        do {
-            s = atomicAdd(&state[j], 0ull);
-            if ((s >> 62) != 0) break;
-            if (++spins > SPIN_LIMIT) {
-                atomicExch(error, 1);
-                return prefix;
-            }
-            __nanosleep(64);
-        } while (true);
-        prefix += s & VALUE_MASK;
-        if ((s >> 62) == 2) break;
-        --j;
-    }
-    return prefix;
-}
 
 __global__ void __launch_bounds__(SCAN_THREADS)
     scan_pairs_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
@@ -103,26 +44,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
     unsigned long long ta, tb;
     unsigned long long ea = block_excl_scan(sa, &ta);
     unsigned long long eb = block_excl_scan(sb, &tb);
-    unsigned long long* state_a = state;
-    unsigned long long* state_b = state + num_tiles;
-    if (threadIdx.x == 0) {
-        if (tile == 0) {
-            atomicExch(&state_a[0], FLAG_INC | ta);
-            atomicExch(&state_b[0], FLAG_INC | tb);
-            prefix_s[0] = 0;
-            prefix_s[1] = 0;
-        } else {
-            atomicExch(&state_a[tile], FLAG_AGG | ta);
-            atomicExch(&state_b[tile], FLAG_AGG | tb);
-            unsigned long long pa = look_back(state_a, tile, error);
-            unsigned long long pb = look_back(state_b, tile, error);
-            __threadfence();
-            atomicExch(&state_a[tile], FLAG_INC | ((pa + ta) & VALUE_MASK));
-            atomicExch(&state_b[tile], FLAG_INC | ((pb + tb) & VALUE_MASK));
-            prefix_s[0] = pa;
-            prefix_s[1] = pb;
-        }
-    }
+    if (threadIdx.x < 32) scan_publish(state, num_tiles, tile, ta, tb, prefix_s, error);
     __syncthreads();
     unsigned long long ra = prefix_s[0] + ea, rb = prefix_s[1] + eb;
 #pragma unroll
@@ -192,15 +114,21 @@ __global__ void narrow_u64_kernel(const uint64_t* in, uint32_t* out, uint32_t n)
 }
 
 __global__ void read_totals_kernel(const uint64_t* a_total, const uint64_t* b_total,
-                                   const uint32_t* words, uint64_t* host_dst) {
+                                   const uint32_t* words, const uint32_t* more,
+                                   uint64_t* host_dst) {
     host_dst[0] = *a_total;
     host_dst[1] = *b_total;
     host_dst[2] = (uint64_t)words[0] | ((uint64_t)words[1] << 32);
+    if (more) {
+        host_dst[3] = (uint64_t)more[0] | ((uint64_t)more[1] << 32);
+        host_dst[4] = (uint64_t)more[2] | ((uint64_t)more[3] << 32);
+    }
 }
 
 cudaError_t launch_read_totals(const uint64_t* a_total, const uint64_t* b_total,
-                               const uint32_t* words, uint64_t* host_dst, cudaStream_t s) {
-    read_totals_kernel<<<1, 1, 0, s>>>(a_total, b_total, words, host_dst);
+                               const uint32_t* words, const uint32_t* more, uint64_t* host_dst,
+                               cudaStream_t s) {
+    read_totals_kernel<<<1, 1, 0, s>>>(a_total, b_total, words, more, host_dst);
     note_launches(1);
     return cudaGetLastError();
 }

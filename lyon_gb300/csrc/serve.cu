@@ -30,8 +30,8 @@
 
 namespace lg {
 int srv_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch, const void* options,
-              uint32_t num_options, const uint32_t* request_first, uint64_t* tv, uint64_t* ti,
-              uint32_t* failed);
+              uint32_t num_options, uint32_t num_verbs, const uint32_t* request_first,
+              uint64_t* tv, uint64_t* ti, uint32_t* failed);
 int srv_configure(lyon_gpu_context* ctx, bool stroke_lane, uint32_t fill_blocks_per_sm,
                   cudaMemPool_t pool);
 int srv_emit(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch, const void* options,
@@ -305,7 +305,8 @@ void run_batch(lyon_srv* s, Worker& w, int kind, std::vector<Request*>& batch, u
     const uint32_t* d_rfirst = w.d_off + 2 * (np + 1);
     uint64_t tv = 0, ti = 0;
     uint32_t failed = 0;
-    int rc = lg::srv_count(w.ctx, kind, &db, w.d_opts, np, d_rfirst, &tv, &ti, &failed);
+    int rc = lg::srv_count(w.ctx, kind, &db, w.d_opts, np, (uint32_t)vc, d_rfirst, &tv, &ti,
+                           &failed);
     if (rc != LYON_OK) {
         finish(s, batch, rc, nullptr, nullptr, nullptr, nullptr, reserved);
         return;

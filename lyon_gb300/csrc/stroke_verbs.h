@@ -1,0 +1,75 @@
+// stroke_verbs.h — launch interface of the verb-parallel stroke (stroke_verbs.cu).
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "kernels.h"
+
+namespace lg {
+
+// Device arrays of the verb-parallel stroke, one entry per verb of the batch ("slot": the verb's
+// index less the batch's first) unless said otherwise. Filled by the count phase, read by the
+// emit phase.
+struct StrokeVerbs {
+    uint32_t cap;          // verbs the arrays have room for (vpre and ipre: one entry more)
+    float4* firsts;        // the verb's first two kept points
+    float4* lasts;         // the kept point before the verb's last one, and the one before that
+    float2* fin;           // its last kept point, where that is not its end point
+    uint32_t* rec;         // first point of the verb; End/Close: the slot of the sub-path's Begin
+    uint32_t* path;
+    uint32_t* join;        // the general join at the verb's end point (packed counts and ids)
+    uint32_t* split;       // the join between the two runs of a verb that has two
+    uint32_t* drops;       // list of verbs whose end point merged (before `split` is written)
+    uint32_t* cut;         // where that join is
+    uint32_t* extra;       // list of the verbs that have one
+    uint32_t* irregular;   // list of the irregular verbs
+    uint32_t* vpre;        // vertices of the batch before this verb (its own until the scan)
+    uint32_t* ipre;        // indices, likewise
+    uint16_t* flags;
+    uint8_t* kind;
+    uint32_t* path_walk;   // per path: not 0 when the path is left to the walk of stroke.cu
+    uint32_t* walk_list;   // those paths
+    uint32_t* path_v;      // per path: vpre and ipre of its first verb
+    uint32_t* path_i;
+    uint32_t* words;       // [0] verbs of the batch, [1] offsets out of order, [2] paths in
+                           // walk_list, [3] some verb has interior steps, [4] drops, [5] scan tile,
+                           // [6] extra, [7] irregular
+    unsigned long long* scan;  // tile states, after the words
+    size_t clear_bytes;    // words and tile states, cleared by every count phase
+};
+constexpr uint32_t STROKE_VERBS_READ = 4;    // words the host reads back
+constexpr uint32_t STROKE_VERBS_WORDS = 16;  // words in all
+// Bytes per verb of the arrays above, for their allocation.
+constexpr size_t STROKE_VERBS_BYTES = 2 * 16 + 8 + 9 * 4 + 2 + 1;
+
+// Streams for kernels that run beside those of the caller's stream: fork(i, s) returns a stream
+// that continues after what is on `s`, join(i, s) makes `s` wait for it. Without streams (none
+// could be made) the work goes on `s` itself.
+struct SideStreams {
+    cudaStream_t stream[2] = {nullptr, nullptr};
+    cudaEvent_t forked[2] = {nullptr, nullptr}, joined[2] = {nullptr, nullptr};
+    cudaStream_t fork(int i, cudaStream_t s) const {
+        if (!stream[i]) return s;
+        cudaEventRecord(forked[i], s);
+        cudaStreamWaitEvent(stream[i], forked[i], 0);
+        return stream[i];
+    }
+    void join(int i, cudaStream_t s) const {
+        if (!stream[i]) return;
+        cudaEventRecord(joined[i], stream[i]);
+        cudaStreamWaitEvent(s, joined[i], 0);
+    }
+};
+
+// Counts of every path (vtx_counts, idx_counts, status of `a`), the paths in walk_list apart.
+// `verbs_hint`: about how many verbs the batch has (sizes the grids only).
+cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
+                                      uint32_t verbs_hint, int num_sms, const SideStreams& side,
+                                      cudaStream_t s);
+// Output of the paths that launch_stroke_verbs_count counted. `runs`: words[3].
+cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
+                                     uint32_t verbs_hint, bool runs, int num_sms,
+                                     const SideStreams& side, cudaStream_t s);
+
+}  // namespace lg
