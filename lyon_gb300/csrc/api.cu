@@ -479,7 +479,7 @@ const lg::SideStreams& side_streams(lyon_gpu_context* ctx) {
     return ctx->side;
 }
 
-// Counts a fixed-width stroke of positions verb by verb. Returns LYON_OK with ctx->verbs_valid
+// Counts a stroke verb by verb. Returns LYON_OK with ctx->verbs_valid
 // false when the batch is left to the path-by-path count (its offsets overlap, or no room for the
 // arrays).
 int count_by_verb(lyon_gpu_context* ctx, const lyon_path_batch* batch,
@@ -536,8 +536,7 @@ int pipeline_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch
     ctx->order_valid = false;
     ctx->split_valid = false;
     ctx->verbs_valid = false;
-    if (kind == KIND_STROKE && n > 0 && !ctx->vw_widths && !ctx->want_sources &&
-        !ctx->vertex_attrs) {
+    if (kind == KIND_STROKE && n > 0) {
         const int r = count_by_verb(ctx, batch, (const lyon_stroke_options*)options, num_options,
                                     index_bits, index_mode, vertex_offset, tv, ti, failed);
         if (r != LYON_OK) return r;

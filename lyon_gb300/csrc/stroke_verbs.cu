@@ -36,145 +36,10 @@
 // and points.
 #include "scan_core.cuh"
 #include "stroke_parts.cuh"
-#include "stroke_verbs.h"
+#include "stroke_verbs.cuh"
 
 namespace lg {
 namespace {
-
-constexpr uint32_t FULL = 0xFFFFFFFFu;
-constexpr int KIND_NONE = 7;           // an unused slot
-constexpr uint32_t KIND_MASK = 7;
-constexpr uint32_t KIND_MNEC = 0x80;   // End/Close: a point merged into the sub-path's first
-constexpr uint32_t KIND_GAP = 0x40;    // line verbs were dropped right before this verb
-// Flags of a verb.
-constexpr uint32_t VF_IRR = 1;         // irregular
-constexpr uint32_t VF_FLAT1 = 2;       // its first kept point is a flattening step
-constexpr uint32_t VF_FLATL = 4;       // the kept point before its last one is one
-constexpr uint32_t VF_NK_SHIFT = 3;    // kept points, at most 3 (two bits)
-constexpr uint32_t VF_TURN = 32;       // a quadratic split at a sharp turn
-constexpr uint32_t VF_TOFIRST = 64;    // its first join's edge ids coincide (EF_SELF_EQ)
-constexpr uint32_t VF_CUT = 128;       // cut in two runs at an interior general join
-constexpr uint32_t VF_MERGED = 256;    // its end point merged: its last kept point is in `fin`
-constexpr uint32_t VF_ENDFLAT = 512;   // and that one is a flattening step
-constexpr uint32_t VF_TWO = VF_TURN | VF_CUT;
-constexpr uint32_t VF_SECOND1 = 1024;  // of two units, the second is one step
-// A curve of more steps than this leaves its path to the walk, which takes 32 steps at a time.
-constexpr uint32_t MAX_SERIAL_STEPS = 1u << 15;
-
-__device__ __forceinline__ bool is_segment(int k) {
-    return k == LYON_VERB_LINE_TO || k == LYON_VERB_QUADRATIC_TO || k == LYON_VERB_CUBIC_TO;
-}
-__device__ __forceinline__ bool is_end(int k) {
-    return k == LYON_VERB_END || k == LYON_VERB_CLOSE;
-}
-__device__ __forceinline__ uint32_t flags_nk(uint32_t f) { return (f >> VF_NK_SHIFT) & 3u; }
-
-// ---- packed joins ---------------------------------------------------------------------------
-// A general join: vertices (21 bits), relative ids the next edge starts from (2 + 2), triangles
-// less vertices + 4 (3 bits: interior triangles less base vertices), whether the edge into it has
-// equal ids. Joins with more vertices or invalid ids are not packed (their path is walked).
-__device__ __forceinline__ bool pack_join(const SlowJoin& j, uint32_t* out) {
-    if (j.st != LYON_OK || j.vcount >= (1u << 21) || j.from_neg_rel > 3u || j.from_pos_rel > 3u ||
-        (j.to_f & ~EF_SELF_EQ) != 0 || j.jtris + 4u < j.vcount || j.jtris + 4u - j.vcount > 7u)
-        return false;
-    *out = j.vcount | (j.from_neg_rel << 21) | (j.from_pos_rel << 23) |
-           ((j.jtris + 4u - j.vcount) << 25) | (j.to_f ? 1u << 28 : 0u);
-    return true;
-}
-__device__ __forceinline__ uint32_t pj_vertices(uint32_t j) { return j & 0x1FFFFFu; }
-__device__ __forceinline__ uint32_t pj_neg(uint32_t j) { return (j >> 21) & 3u; }
-__device__ __forceinline__ uint32_t pj_pos(uint32_t j) { return (j >> 23) & 3u; }
-__device__ __forceinline__ uint32_t pj_tris(uint32_t j) {
-    return pj_vertices(j) + ((j >> 25) & 7u) - 4u;
-}
-__device__ __forceinline__ uint32_t pj_to(uint32_t j) { return (j >> 28) & 1u ? EF_SELF_EQ : 0u; }
-__device__ __forceinline__ uint32_t pj_from(uint32_t j) {
-    return pj_neg(j) == pj_pos(j) ? EF_SELF_EQ : 0u;
-}
-
-// A flattening step's join, packed.
-constexpr uint32_t PACKED_STEP = 2u | (1u << 21) | (2u << 25);
-
-// ---- a verb's curve units ---------------------------------------------------------------------
-struct Unit {
-    Poly p;
-    V2 to;
-    float s, t0;  // lyon's step 1/n and the parameter the unit starts from
-    uint32_t m;   // steps (the last one is `to`); 0: no such unit
-};
-
-__device__ __forceinline__ void unit_of(Unit& u, const Poly& p, V2 to, float n) {
-    u.p = p;
-    u.to = to;
-    u.s = 1.0f / n;
-    u.t0 = 0.0f;
-    u.m = to_u32_or1(n);
-}
-__device__ __forceinline__ float unit_t(const Unit& u, uint32_t k) {
-    return accumulate_t(u.s, 0, u.t0, k);
-}
-// Its first point, and the point before its last one (`from` when it is one step).
-__device__ __forceinline__ V2 first_point(const Unit& u) {
-    return u.m >= 2 ? poly_sample(u.p, u.t0 + u.s) : u.to;
-}
-__device__ __forceinline__ V2 point_before_end(const Unit& u, V2 from) {
-    return u.m >= 2 ? poly_sample(u.p, unit_t(u, u.m - 1)) : from;
-}
-
-// The one or two units of a segment verb, with lyon's arithmetic (setup_verb, stroke_parts.cuh).
-// `cut`: the parameter of a sharp turn (VF_TURN), or for a verb that is cut (VF_CUT) the step of
-// the join between its runs and, in the upper 16 bits, how many steps merge into that point.
-__device__ __forceinline__ void verb_units(int kind, uint32_t p, const float* points, float tol,
-                                           uint32_t flags, uint32_t cut, Unit& a, Unit& b) {
-    b.m = 0;
-    if (kind == LYON_VERB_LINE_TO) {
-        a.to = load_pt(points, p);
-        a.m = 1;
-        a.s = 1.0f;
-        a.t0 = 0.0f;
-        return;
-    }
-    const V2 from = load_pt(points, p - 1);
-    if (kind == LYON_VERB_QUADRATIC_TO) {
-        const V2 ctrl = load_pt(points, p), to = load_pt(points, p + 1);
-        if (flags & VF_TURN) {
-            const float ts = __uint_as_float(cut);
-            const V2 sp = quad_sample(from, ctrl, to, ts);
-            const V2 bc = lerp(from, ctrl, ts), ac = lerp(ctrl, to, ts);
-            unit_of(a, quad_poly(from, bc, sp), sp, quad_wang(from, bc, sp, tol));
-            unit_of(b, quad_poly(sp, ac, to), to, quad_wang(sp, ac, to, tol));
-            return;
-        }
-        unit_of(a, quad_poly(from, ctrl, to), to, quad_wang(from, ctrl, to, tol));
-    } else {
-        const V2 c1 = load_pt(points, p), c2 = load_pt(points, p + 1), to = load_pt(points, p + 2);
-        unit_of(a, cubic_poly(from, c1, c2, to), to, cubic_wang(from, c1, c2, to, tol));
-    }
-    if (flags & VF_CUT) {
-        const uint32_t at = cut & 0xFFFFu, gap = cut >> 16;
-        const float t = unit_t(a, at);
-        b = a;
-        b.m = a.m - at - gap;
-        b.t0 = accumulate_t(a.s, at, t, at + gap);
-        a.m = at;
-        a.to = poly_sample(a.p, t);
-    }
-}
-
-// The end point of the verb in `slot` (a Begin or a segment).
-__device__ __forceinline__ V2 end_point(const StrokeVerbs& S, const float* points, uint32_t slot) {
-    const int k = S.kind[slot] & KIND_MASK;
-    return load_pt(points, S.rec[slot] + points_of_verb(k) - 1);
-}
-// Its last kept point, once walk_kernel has run: the end point, or the step it merged into.
-__device__ __forceinline__ V2 last_kept(const StrokeVerbs& S, const float* points, uint32_t slot) {
-    const int k = S.kind[slot] & KIND_MASK;
-    if (k != LYON_VERB_BEGIN && (S.flags[slot] & VF_MERGED)) {
-        const float2 f = S.fin[slot];
-        return V2{f.x, f.y};
-    }
-    return load_pt(points, S.rec[slot] + points_of_verb(k) - 1);
-}
 
 // The skip test of flattened_step (stroke.rs:1778-1782) cannot fire at a join whose edge into it is
 // longer than this bound, when the previous join's side points are symmetric (see stroke.cu).
@@ -191,15 +56,6 @@ __device__ __forceinline__ bool skip_fires(V2 prv, V2 pn, V2 nn, V2 cur, V2 nxt,
     const SidePair s = fast_join_sides(prv, cur, nxt, hw);
     const V2 pe = cur - prv;
     return dot(pe, s.pn - pn) < 0.0f && dot(pe, s.nn - nn) < 0.0f;
-}
-
-__device__ __forceinline__ void leave_to_walk(const StrokeVerbs& S, uint32_t path) {
-    S.path_walk[path] = 1u;
-}
-
-__device__ __forceinline__ uint32_t batch_verbs(const StrokeArgs& A) {
-    const uint32_t a = A.verb_offsets[0], b = A.verb_offsets[A.num_paths];
-    return b >= a ? b - a : 0u;
 }
 
 // ---- 1. prepare --------------------------------------------------------------------------------
@@ -1401,7 +1257,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) verb_scan_kernel(StrokeArgs A, S
             if ((is_segment(kind) || is_end(kind)) && !S.path_walk[S.path[v]]) {
                 a = S.vpre[v];
                 b = S.ipre[v];
-                if (is_segment(kind) && (S.kind[v - 1] & KIND_MASK) != LYON_VERB_BEGIN) {
+                if (!A.widths && is_segment(kind) &&
+                    (S.kind[v - 1] & KIND_MASK) != LYON_VERB_BEGIN) {
                     const uint32_t f = S.flags[v];
                     if (flags_nk(f) >= 2 || is_segment(S.kind[v + 1] & KIND_MASK))
                         b += 3u * edge_count_flags(pj_from(S.join[v - 1]),
@@ -1740,21 +1597,28 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
     walk_kernel<<<grid_for(verbs_hint, WIN_WARPS, num_sms, 8), WIN_WARPS * 32,
                   WIN_WARPS * sizeof(WalkSmem), s>>>(a, v);
     drops_kernel<<<grid_for(0, 128, num_sms, 1), 128, 0, s>>>(a, v);
-    // Tails read the points beside the sub-paths' ends and nothing of the joins.
-    const cudaStream_t t = side.fork(0, s);
-    tails_kernel<false><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
-    extra_count_kernel<<<grid_for(verbs_hint / 8, 128, num_sms, 8), 128, 0, s>>>(a, v);
-    joins_count_kernel<<<by_verb, 256, 0, s>>>(a, v);
-    side.join(0, s);
+    if (a.widths) {
+        launch_stroke_steps_count(a, v, verbs_hint, num_sms, s);
+    } else {
+        // Tails read the points beside the sub-paths' ends and nothing of the joins.
+        const cudaStream_t t = side.fork(0, s);
+        tails_kernel<false><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
+        extra_count_kernel<<<grid_for(verbs_hint / 8, 128, num_sms, 8), 128, 0, s>>>(a, v);
+        joins_count_kernel<<<by_verb, 256, 0, s>>>(a, v);
+        side.join(0, s);
+        note_launches(3);
+    }
     verb_scan_kernel<<<grid_for(verbs_hint, SCAN_TILE, num_sms, 4), SCAN_THREADS, 0, s>>>(a, v);
     paths_kernel<<<grid_for(n, 256, num_sms, 8), 256, 0, s>>>(a, v);
-    note_launches(9);
+    note_launches(6);
     return cudaGetLastError();
 }
 
 cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
                                      uint32_t verbs_hint, bool runs, int num_sms,
                                      const SideStreams& side, cudaStream_t s) {
+    if (a.widths || a.sources || a.vertex_attrs)
+        return launch_stroke_steps_emit(a, v, verbs_hint, num_sms, s);
     // The three write different parts of the output; joins and tails are short of warps and of
     // threads that agree, and fill the gaps of the runs.
     const cudaStream_t j = side.fork(0, s), t = side.fork(1, s);

@@ -227,3 +227,90 @@ def test_offsets_from_the_middle_of_a_batch(ctx):
     a = by_walk(ctx, db, od, 23, 32, T.INDEX_GLOBAL)
     b = by_verb(ctx, db, od, 23, 32, T.INDEX_GLOBAL)
     assert all(np.array_equal(a[k], b[k]) for k in ("st", "vo", "io", "i", "v"))
+
+
+# ---- attribute records, variable widths and vertex sources ----------------------------------------
+
+def stepped(ctx, batch, opts, how, by_path=False, bits=32, mode=T.INDEX_GLOBAL):
+    """One call of the stepped outputs. With `by_path` a last path whose offsets run backwards (it
+    strokes to nothing) makes the whole batch go path by path."""
+    import torch
+    vo, po = batch.verb_offsets, batch.point_offsets
+    if by_path:
+        vo, po = np.append(vo, vo[-1] - 1), np.append(po, po[-1])
+        opts = np.append(opts, opts[-1:]) if len(opts) > 1 else opts
+    b = PathBatch(batch.verbs, batch.points, vo.astype(np.uint32), po.astype(np.uint32))
+    db, od = T.DeviceBatch.upload(b, 0), T.upload_options(opts, 0)
+    rng = np.random.default_rng(5)
+    w = torch.from_numpy(rng.uniform(0.3, 2.5, len(b.points)).astype(np.float32)).cuda()
+    attrs = torch.from_numpy(rng.uniform(0.5, 2, (len(b.points), 3)).astype(np.float32)).cuda()
+    kw = {"records": dict(attributes=True), "widths": dict(widths=w),
+          "widths records": dict(widths=w, attributes=True),
+          "sources": dict(custom_attributes=attrs),
+          "sources records": dict(custom_attributes=attrs, attributes=True),
+          "sources widths": dict(custom_attributes=attrs, width_attribute=1),
+          "sources widths records": dict(custom_attributes=attrs, width_attribute=2,
+                                         attributes=True)}[how]
+    torch.cuda.synchronize()
+    res = T.tessellate_paths("stroke", db, od, len(opts), bits, mode, 0, ctx, **kw)
+    ctx.synchronize()
+    n = batch.num_paths
+    out = {"st": res.statuses().cpu().numpy()[:n], "failed": np.array(res.num_failed_paths)}
+    o = res.offsets()
+    out["vo"], out["io"] = o[0].cpu().numpy()[:n + 1], o[1].cpu().numpy()[:n + 1]
+    if res.total_vertices:
+        v = res.records() if "records" in how else res.vertices()
+        out["v"] = v.cpu().numpy()
+        if "sources" in how:
+            out["src"] = res.sources().cpu().numpy()
+            out["attr"] = res.custom_attributes().cpu().numpy()
+    if res.total_indices:
+        out["i"] = res.indices().cpu().numpy()
+    return out
+
+
+def same_bits(a, b):
+    assert a.keys() == b.keys()
+    for k in a:
+        x, y = a[k], b[k]
+        assert x.shape == y.shape, (k, x.shape, y.shape)
+        if x.dtype == np.float32:
+            nan = np.isnan(x)
+            assert np.array_equal(nan, np.isnan(y)), k
+            x, y = x[~nan].view(np.uint32), y[~nan].view(np.uint32)
+        assert np.array_equal(x, y), (k, np.nonzero(x != y)[0][:8])
+
+
+STEPPED = ["records", "widths", "widths records", "sources", "sources records", "sources widths",
+           "sources widths records"]
+
+
+@pytest.mark.parametrize("how", STEPPED)
+@pytest.mark.parametrize("join", [None, 0, 1, 2, 3])
+def test_stepped_rough_paths(ctx, how, join):
+    for seed in (11, 12):
+        batch = rough_paths(500, seed)
+        o = options(np.random.default_rng(seed), batch.num_paths, join=join)
+        o["line_width"] = np.maximum(o["line_width"], 0.3)
+        same_bits(stepped(ctx, batch, o, how, by_path=True), stepped(ctx, batch, o, how))
+
+
+@pytest.mark.parametrize("how", STEPPED)
+def test_stepped_scenes(ctx, how):
+    batch, o = workloads.batched_stroke(600, seed=41)
+    o["line_join"] = np.arange(len(o)) % 4
+    o["start_cap"] = np.arange(len(o)) % 3
+    o["tolerance"] = 0.1
+    same_bits(stepped(ctx, batch, o, how, by_path=True), stepped(ctx, batch, o, how))
+    batch, o = workloads.map_polylines(1500, seed=42, max_len=300)
+    same_bits(stepped(ctx, batch, o, how, by_path=True, bits=16, mode=T.INDEX_PER_PATH),
+              stepped(ctx, batch, o, how, bits=16, mode=T.INDEX_PER_PATH))
+
+
+@pytest.mark.parametrize("n", [1, 2, 33])
+def test_stepped_small_batches(ctx, n):
+    for how in STEPPED:
+        batch = rough_paths(n, 90 + n, max_verbs=120)
+        o = options(np.random.default_rng(n), 1, tol=0.05)
+        o["line_width"] = 3.0
+        same_bits(stepped(ctx, batch, o, how, by_path=True), stepped(ctx, batch, o, how))
