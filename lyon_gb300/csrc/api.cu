@@ -1874,7 +1874,7 @@ int lyon_gpu_flatten_counts(lyon_gpu_context* ctx, const lyon_path_batch* batch,
     a.tolerance = tolerance;
     a.counts = counts;
     return set_err(ctx, "flatten counts",
-                   lg::launch_flatten(a, false, ctx->num_sms * 8, ctx->stream))
+                   lg::launch_flatten_counts(a, ctx->num_sms, ctx->stream))
                ? LYON_OK
                : LYON_ERR_CUDA;
 }
@@ -2096,12 +2096,25 @@ int lyon_gpu_flatten_paths(lyon_gpu_context* ctx, const lyon_path_batch* batch, 
             return LYON_ERR_CUDA;
         nv = *reinterpret_cast<uint32_t*>(ctx->h_small.ptr);
     }
-    if (!ensure(ctx, ctx->flat_counts, (size_t)nv * 4 + 16) ||
+    if (!ensure(ctx, ctx->flat_counts, (size_t)nv * 8 + 16) ||
         !ensure(ctx, ctx->flat_offsets, ((size_t)nv + 1) * 8 * 2 + 16) ||
         !ensure(ctx, ctx->scan_state, 2 * lg::scan_tile_count(nv) * 8 + 16))
         return LYON_ERR_OUT_OF_MEMORY;
-    int r = lyon_gpu_flatten_counts(ctx, batch, tolerance, as<uint32_t>(ctx->flat_counts));
-    if (r != LYON_OK) return r;
+    lg::FlattenArgs a;
+    memset(&a, 0, sizeof a);
+    a.verbs = batch->verbs;
+    a.points = batch->points;
+    a.verb_offsets = batch->verb_offsets;
+    a.point_offsets = batch->point_offsets;
+    a.num_paths = batch->num_paths;
+    a.tolerance = tolerance;
+    a.counts = as<uint32_t>(ctx->flat_counts);
+    a.firsts = a.counts + nv;
+    // Verbs of no path (before the first offset) have no points.
+    cudaMemsetAsync(a.firsts, 0xFF, (size_t)nv * 4, s);
+    if (batch->num_paths > 0 &&
+        !set_err(ctx, "flatten counts", lg::launch_flatten_counts(a, ctx->num_sms, s)))
+        return LYON_ERR_CUDA;
     uint64_t* offs = as<uint64_t>(ctx->flat_offsets);
     uint64_t* offs2 = offs + nv + 1;
     uint32_t* sw = small_words(ctx);
@@ -2116,18 +2129,10 @@ int lyon_gpu_flatten_paths(lyon_gpu_context* ctx, const lyon_path_batch* batch, 
     if (!set_err(ctx, "sync", cudaStreamSynchronize(s))) return LYON_ERR_CUDA;
     uint64_t total = *reinterpret_cast<uint64_t*>(ctx->h_small.ptr);
     if (!ensure(ctx, ctx->flat_points, total * 8 + 16)) return LYON_ERR_OUT_OF_MEMORY;
-    lg::FlattenArgs a;
-    memset(&a, 0, sizeof a);
-    a.verbs = batch->verbs;
-    a.points = batch->points;
-    a.verb_offsets = batch->verb_offsets;
-    a.point_offsets = batch->point_offsets;
-    a.num_paths = batch->num_paths;
-    a.tolerance = tolerance;
     a.offsets = offs;
     a.out_points = as<float>(ctx->flat_points);
     if (batch->num_paths > 0 &&
-        !set_err(ctx, "flatten points", lg::launch_flatten(a, true, ctx->num_sms * 8, s)))
+        !set_err(ctx, "flatten points", lg::launch_flatten_points(a, nv, ctx->num_sms, s)))
         return LYON_ERR_CUDA;
     *out_points = as<float>(ctx->flat_points);
     *out_offsets = reinterpret_cast<uint32_t*>(offs2);

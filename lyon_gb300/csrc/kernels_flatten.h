@@ -16,10 +16,17 @@ struct FlattenArgs {
     uint32_t num_paths;
     float tolerance;
     uint32_t* counts;          // one per verb (count pass)
+    uint32_t* firsts;          // one per verb: its first point (count pass; null: not wanted), or
+                               // FLATTEN_NO_POINTS
     const uint64_t* offsets;   // exclusive scan of counts (point pass)
     float* out_points;         // point pass output
 };
 
-cudaError_t launch_flatten(const FlattenArgs& a, bool write_points, int grid, cudaStream_t s);
+constexpr uint32_t FLATTEN_NO_POINTS = 0xFFFFFFFFu;
+
+cudaError_t launch_flatten_counts(const FlattenArgs& a, int num_sms, cudaStream_t s);
+// Points of the verbs [0, num_verbs) that the count pass gave a first point.
+cudaError_t launch_flatten_points(const FlattenArgs& a, uint32_t num_verbs, int num_sms,
+                                  cudaStream_t s);
 
 }  // namespace lg

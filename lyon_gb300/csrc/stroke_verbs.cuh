@@ -2,13 +2,13 @@
 // verb: its flags, its curve units and the packed form of a general join.
 #pragma once
 
+#include "points.cuh"
 #include "stroke_parts.cuh"
 #include "stroke_verbs.h"
 
 namespace lg {
 namespace {
 
-constexpr uint32_t FULL = 0xFFFFFFFFu;
 constexpr int KIND_NONE = 7;           // an unused slot
 constexpr uint32_t KIND_MASK = 7;
 constexpr uint32_t KIND_MNEC = 0x80;   // End/Close: a point merged into the sub-path's first
@@ -63,23 +63,6 @@ __device__ __forceinline__ uint32_t pj_from(uint32_t j) {
 constexpr uint32_t PACKED_STEP = 2u | (1u << 21) | (2u << 25);
 
 // ---- a verb's curve units ---------------------------------------------------------------------
-struct Unit {
-    Poly p;
-    V2 to;
-    float s, t0;  // lyon's step 1/n and the parameter the unit starts from
-    uint32_t m;   // steps (the last one is `to`); 0: no such unit
-};
-
-__device__ __forceinline__ void unit_of(Unit& u, const Poly& p, V2 to, float n) {
-    u.p = p;
-    u.to = to;
-    u.s = 1.0f / n;
-    u.t0 = 0.0f;
-    u.m = to_u32_or1(n);
-}
-__device__ __forceinline__ float unit_t(const Unit& u, uint32_t k) {
-    return accumulate_t(u.s, 0, u.t0, k);
-}
 // Its first point, and the point before its last one (`from` when it is one step).
 __device__ __forceinline__ V2 first_point(const Unit& u) {
     return u.m >= 2 ? poly_sample(u.p, u.t0 + u.s) : u.to;
