@@ -1,15 +1,11 @@
-// fill.cu — batched fill tessellation: lyon's sweep-line FillTessellator, one thread per path
-// (several per warp).
+// fill.cu — batched fill tessellation: lyon's sweep-line FillTessellator, one warp per path.
 //
 // Pipeline (per batched call):
-//   1. fill_sweep_kernel: a persistent grid of sweeper threads (several per warp) takes paths
-//      from an atomic counter. Each sweeper builds the path's event queue (event_queue.rs:
-//      441-905: downward-oriented edges, curves flattened with their t ranges, vertex events
-//      at local maxima), sorts it with lyon's linked-list merge sort (event_queue.rs:301-384,
-//      same recursion so equal positions form the same sibling chains), runs the sweep
-//      (fill.rs:749-2151) and the monotone tessellators (monotone.rs), writing vertices and
-//      triangles (path-relative ids) into its private heap; at the end it reserves room in a
-//      staging pool with one atomic add and copies them there.
+//   1. fill_warp_kernel: a persistent grid of warps takes paths from an atomic counter, the bigger
+//      ones first. A warp builds its path's event queue, sorts it, runs the sweep and triangulates
+//      the spans (fill_warp.cuh) in its private heap; at the end it reserves room in a staging
+//      pool with one atomic add per array and writes vertices and triangles (path-relative ids)
+//      there. Large batches' tiny paths go to fill_sweep_kernel, a thread each (fill_sweep.cuh).
 //   2. the caller's index-range check and look-back scan turn the per-path counts into offsets;
 //   3. fill_emit_kernel: one warp per path copies the staged vertices to their final place and
 //      the indices with the path's id base added (u16 or u32).
@@ -23,6 +19,7 @@
 #include "fill.h"
 #include "kernels.h"
 #include "fill_sweep.cuh"
+#include "fill_warp.cuh"
 
 namespace lg {
 namespace fillk {
@@ -35,20 +32,46 @@ constexpr int32_t STATUS_RETRY = -1;
 #ifndef LG_FILL_MIN_BLOCKS
 #define LG_FILL_MIN_BLOCKS 16
 #endif
-#ifndef LG_FILL_LANES
-#define LG_FILL_LANES 12
-#endif
-// 32-thread blocks per SM; the first `lanes` threads of each block are sweepers, each with its
-// own path and heap: as many lanes as the launch has paths per block (rounded down), between 1
-// and LG_FILL_LANES (LYON_GB300_FILL_LANES forces a lane count, 1 to 32, for every launch). On
-// 200,000 glyph paths the non-zero sweep took 1800 / 1717 / 1551 / 1643 / 2400 ms with 1 / 4 /
-// 8 / 16 / 32 lanes at 32 blocks per SM (64 registers, small spills): diverged lanes run one
-// after another, so more than 8 loses again. With 96 registers and no spills, 20 blocks per SM
-// took 1462 / 1491 / 1443 ms with 8 / 12 / 16 lanes, 24 blocks (80 registers) 1442 ms with 8,
-// and 16 blocks 1487 / 1310 ms with 8 / 12 lanes (192 sweepers per SM, 7.5 GB of heaps).
+// One-warp blocks per SM, a path each.
 constexpr uint32_t FILL_SWEEPERS_PER_SM = LG_FILL_SWEEPERS_PER_SM;
 // Heaps of all sweepers together stay under this many bytes (fewer blocks when larger).
 constexpr size_t FILL_HEAP_POOL_BYTES = 16ull << 30;
+
+// Paths of lines only with fewer than TINY_POINTS points, when there are TINY_MIN_PATHS of them or
+// more, are swept by a thread each (fill_sweep.cuh), TINY_LANES of a warp's. A warp's sweep of such a
+// path is mostly what every path costs (its arrays, the steps around each event), and that code goes
+// through the instruction cache once per path: a thread per path shares each fetch. Microseconds for
+// a batch by warps and by threads: triangles 20,000 248 and 180, 80,000 730 and 379, 200,000 1708 and
+// 854; quadrilaterals 10,000 186 and 216, 20,000 305 and 258, 200,000 2392 and 1795; hexagons 80,000
+// 1295 and 1207; octagons 80,000 1662 and 1695, 200,000 4106 and 4368. Of 1, 4, 8, 12, 16 and 32
+// threads of a warp 12 were fastest.
+constexpr uint32_t TINY_POINTS = 8;  // a power of two: a bin of the size order
+constexpr uint32_t TINY_MIN_PATHS = 16384;
+constexpr uint32_t TINY_LANES = 12;
+
+// Of the size order's counters: the number of paths with fewer than TINY_POINTS points.
+__device__ __forceinline__ uint32_t tiny_paths(const uint32_t* counters) {
+    uint32_t n = 0;
+    for (uint32_t b = 32u - 3u; b < SIZE_ORDER_BINS; ++b) n += counters[b];
+    return n;
+}
+static_assert(TINY_POINTS == 1u << 3, "bins 29 and up hold paths of fewer than 8 points");
+
+// Sizes for the size order: points, at least TINY_POINTS for a path with a curve.
+__global__ void fill_sizes_kernel(const uint8_t* verbs, const uint32_t* verb_offsets,
+                                  const uint32_t* point_offsets, uint32_t n, uint32_t* sizes) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t size = point_offsets[i + 1] - point_offsets[i];
+    if (size < TINY_POINTS) {
+        const uint32_t v0 = verb_offsets[i], v1 = verb_offsets[i + 1];
+        bool tiny = v1 - v0 <= 2 * TINY_POINTS;
+        for (uint32_t v = v0; tiny && v < v1; ++v)
+            tiny = verbs[v] != LYON_VERB_QUADRATIC_TO && verbs[v] != LYON_VERB_CUBIC_TO;
+        if (!tiny) size = TINY_POINTS;
+    }
+    sizes[i] = size;
+}
 
 struct SweepArgs {
     const uint8_t* verbs;
@@ -59,8 +82,12 @@ struct SweepArgs {
     uint32_t num_options;
     const uint32_t* order;  // null: item = path
     uint32_t num_items;
-    uint32_t lanes;         // sweepers per block (its first threads)
-    uint32_t* counters;     // [0] work, [1] retry count, [2] paths whose heap ran out
+    // [0] work, [1] retry count, [2] paths whose heap ran out, [3] work of the threads
+    uint32_t* counters;
+    // The size order's counters when tiny paths may be swept by threads, else null.
+    const uint32_t* size_counters;
+    uint32_t thread_heap_words;
+    uint32_t lanes;  // threads of a block that sweep tiny paths (its first)
     unsigned long long* stage_tops;  // [0] vertices, [1] indices
     uint32_t* heaps;
     uint32_t heap_words;
@@ -82,17 +109,95 @@ struct SweepArgs {
 };
 
 template <bool SRC>
+__global__ void __launch_bounds__(32, LG_FILL_MIN_BLOCKS) fill_warp_kernel(SweepArgs A) {
+    __shared__ SweepSmem smem;
+    const uint32_t lane = threadIdx.x;
+    WarpFiller<SRC> f(smem);
+    uint32_t* heap = A.heaps + (size_t)blockIdx.x * A.heap_words;
+    const uint32_t tiny = A.size_counters ? tiny_paths(A.size_counters) : 0u;
+    const uint32_t num_items = A.num_items - (tiny >= TINY_MIN_PATHS ? tiny : 0u);
+    for (;;) {
+        uint32_t item = 0;
+        if (lane == 0) item = atomicAdd(&A.counters[0], 1u);
+        item = __shfl_sync(FULL, item, 0);
+        if (item >= num_items) break;
+        const uint32_t path = A.order ? A.order[item] : item;
+        const uint32_t v0 = A.verb_offsets[path], v1 = A.verb_offsets[path + 1];
+        const uint32_t p0 = A.point_offsets[path], p1 = A.point_offsets[path + 1];
+        const lyon_fill_options o = A.options[A.num_options > 1 ? path : 0];
+        f.sweep(heap, A.heap_words, A.verbs + v0, v1 - v0, A.points + 2 * (size_t)p0, p1 - p0, o);
+        uint32_t nv = 0, ni = 0, ns = 0;
+        if (f.err == LYON_OK) {
+            ni = 3 * f.prepare_triangles();
+            nv = f.out_n;
+            ns = f.src_n;
+        }
+        int32_t st = f.err;
+        if (st == LYON_OK) {
+            unsigned long long vb = 0, ib = 0, sb = 0;
+            if (lane == 0) {
+                vb = atomicAdd(&A.stage_tops[0], (unsigned long long)nv);
+                ib = atomicAdd(&A.stage_tops[1], (unsigned long long)ni);
+                if (SRC) sb = atomicAdd(&A.stage_tops[2], (unsigned long long)ns);
+            }
+            vb = __shfl_sync(FULL, vb, 0);
+            ib = __shfl_sync(FULL, ib, 0);
+            sb = __shfl_sync(FULL, sb, 0);
+            if (vb + nv > A.stage_v_cap || ib + ni > A.stage_i_cap ||
+                (SRC && sb + ns > A.stage_s_cap)) {
+                st = STATUS_RETRY;
+            } else {
+                if (SRC) {
+                    for (uint32_t i = lane; i < 3 * ns; i += 32)
+                        A.stage_s[3 * sb + i] = smem.out_src[i];
+                    for (uint32_t i = lane; i < nv; i += 32)
+                        A.stage_sfirst[vb + i] = smem.out_sfirst[i];
+                    if (lane == 0) A.stage_soff[path] = sb;
+                }
+                for (uint32_t i = lane; i < nv; i += 32)
+                    A.stage_v[vb + i] = make_float2(smem.out_v[i].x, smem.out_v[i].y);
+                f.write_triangles(A.stage_i + ib);
+                if (lane == 0) {
+                    A.stage_off[2 * (size_t)path] = vb;
+                    A.stage_off[2 * (size_t)path + 1] = ib;
+                }
+            }
+        } else if (st == FILL_ERR_HEAP) {
+            st = STATUS_RETRY;
+            if (lane == 0) atomicAdd(&A.counters[2], 1u);
+        }
+        if (lane == 0) {
+            if (st == STATUS_RETRY) {
+                if (A.final_attempt) {
+                    st = LYON_ERR_CAPACITY;
+                } else {
+                    const uint32_t r = atomicAdd(&A.counters[1], 1u);
+                    A.retry_list[r] = path;
+                }
+            }
+            A.vtx_counts[path] = st == LYON_OK ? nv : 0u;
+            A.idx_counts[path] = st == LYON_OK ? ni : 0u;
+            if (SRC) A.src_counts[path] = st == LYON_OK ? ns : 0u;
+            A.status[path] = st;
+        }
+        __syncwarp();
+    }
+}
+
+template <bool SRC>
 __global__ void __launch_bounds__(32, LG_FILL_MIN_BLOCKS) fill_sweep_kernel(SweepArgs A) {
     // Each of the block's first `lanes` threads sweeps its own paths with its own heap. The
     // sweep's control flow depends on the path, so lanes diverge; where they run the same code
     // (the event loop's common steps) one instruction fetch serves several paths.
-    if (threadIdx.x >= A.lanes) return;
+    const uint32_t tiny = A.size_counters ? tiny_paths(A.size_counters) : 0u;
+    if (threadIdx.x >= A.lanes || tiny < TINY_MIN_PATHS) return;
+    const uint32_t first = A.num_items - tiny;
     const uint32_t wid = blockIdx.x * A.lanes + threadIdx.x;
     FillerT<SRC> f;
-    f.h.w = A.heaps + (size_t)wid * A.heap_words;
-    f.h.cap = A.heap_words;
+    f.h.w = A.heaps + (size_t)wid * A.thread_heap_words;
+    f.h.cap = A.thread_heap_words;
     for (;;) {
-        const uint32_t item = atomicAdd(&A.counters[0], 1u);
+        const uint32_t item = first + atomicAdd(&A.counters[3], 1u);
         if (item >= A.num_items) break;
         const uint32_t path = A.order ? A.order[item] : item;
         const uint32_t v0 = A.verb_offsets[path], v1 = A.verb_offsets[path + 1];
@@ -129,8 +234,7 @@ __global__ void __launch_bounds__(32, LG_FILL_MIN_BLOCKS) fill_sweep_kernel(Swee
                 A.stage_off[2 * (size_t)path + 1] = ib;
             }
         } else if (st == FILL_ERR_HEAP) {
-            st = STATUS_RETRY;
-            atomicAdd(&A.counters[2], 1u);
+            st = STATUS_RETRY;  // by a warp, whose heap is larger
         }
         if (st == STATUS_RETRY) {
             if (A.final_attempt) {
@@ -257,14 +361,14 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
         reinterpret_cast<char*>(fb.work) + 16);
     uint32_t* lists[2] = {reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(fb.work) + 64),
                           reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(fb.work) + 64) + n};
-    // Sweepers (one per warp) and heaps; heaps start at 64 K words (256 KB), which covers nearly
-    // every glyph-sized path.
+    // Sweepers (one warp each) and heaps; heaps start at 128 K words (512 KB), which covers paths of
+    // about 4,000 events.
     const uint32_t per_sm =
         fb.blocks_per_sm_cap > 0 && fb.blocks_per_sm_cap < (uint32_t)fillk::FILL_SWEEPERS_PER_SM
             ? fb.blocks_per_sm_cap
             : (uint32_t)fillk::FILL_SWEEPERS_PER_SM;
     const uint32_t threads = (uint32_t)(num_sms > 0 ? num_sms : 1) * per_sm;
-    if (fb.heap_words == 0) fb.heap_words = 65536;
+    if (fb.heap_words == 0) fb.heap_words = 131072;
     // Staging: start from a guess of 4 vertices and 12 indices per input point.
     if (fb.stage_v_cap == 0) {
         uint32_t npts = 0;
@@ -287,35 +391,34 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
         if (error) *error = "cudaMalloc (fill source staging)";
         return LYON_ERR_OUT_OF_MEMORY;
     }
-    cudaMemsetAsync(tops, 0, 24, stream);
     // Big paths first, so that the last paths a sweeper takes are short ones and the launch
     // does not end on one long sweep. The order lives in the second retry list, which the first
     // attempt does not write.
     uint32_t* size_counters = lists[1] + n;
     uint8_t* size_cls = reinterpret_cast<uint8_t*>(size_counters + 2 * SIZE_ORDER_BINS);
     const uint32_t* order = nullptr;
-    if (launch_size_order(batch->point_offsets, n, size_cls, lists[1], size_counters, stream) ==
-        cudaSuccess)
+    const bool tiny = n >= fillk::TINY_MIN_PATHS;
+    if (tiny) {  // (the sizes lie in the first retry list, which is written after the order)
+        fillk::fill_sizes_kernel<<<(n + 255) / 256, 256, 0, stream>>>(
+            batch->verbs, batch->verb_offsets, batch->point_offsets, n, lists[0]);
+        lg::note_launches(1);
+    }
+    if (launch_size_order(batch->point_offsets, n, size_cls, lists[1], size_counters, stream,
+                          tiny ? lists[0] : nullptr) == cudaSuccess)
         order = lists[1];
     uint32_t items = n;
-    uint32_t max_lanes = LG_FILL_LANES;
-    bool forced = false;
-    if (fb.lanes >= 1 && fb.lanes <= 32) max_lanes = fb.lanes, forced = true;
+    // Threads of a block that sweep tiny paths: as many as the launch has paths per block, up to
+    // TINY_LANES (LYON_GB300_FILL_LANES or the context's setting force a number, 1 to 32).
+    uint32_t lanes = std::max<uint32_t>(1u, std::min<uint32_t>(fillk::TINY_LANES, n / threads));
+    if (fb.lanes >= 1 && fb.lanes <= 32) lanes = fb.lanes;
     if (const char* env = getenv("LYON_GB300_FILL_LANES")) {
         const long v = strtol(env, nullptr, 10);
-        if (v >= 1 && v <= 32) max_lanes = (uint32_t)v, forced = true;
+        if (v >= 1 && v <= 32) lanes = (uint32_t)v;
     }
     const int MAX_ATTEMPTS = 4;
     for (int attempt = 0; attempt < MAX_ATTEMPTS; ++attempt) {
         uint32_t nthreads = threads;
-        // A lane shares its warp's issue slots with the other lanes, so a path on a shared warp
-        // takes longer than alone: lanes are added only when there are two or more paths per
-        // block (large batches, for throughput), never for a small launch (a served request, the
-        // retry of a few paths), whose latency is one path's sweep.
-        uint32_t lanes = forced ? max_lanes
-                                : std::max<uint32_t>(1u, std::min<uint32_t>(max_lanes,
-                                                                            items / nthreads));
-        size_t heap_bytes = (size_t)fb.heap_words * 4 * nthreads * lanes;
+        size_t heap_bytes = (size_t)fb.heap_words * 4 * nthreads;
         // Keep the heaps under the pool size: fewer blocks when each heap is large.
         while (heap_bytes > fillk::FILL_HEAP_POOL_BYTES && nthreads > 4) {
             nthreads /= 2;
@@ -325,7 +428,8 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
             if (error) *error = "cudaMalloc (fill heaps)";
             return LYON_ERR_OUT_OF_MEMORY;
         }
-        cudaMemsetAsync(counters, 0, 12, stream);
+        // (the staging tops, behind the counters, only at the start)
+        cudaMemsetAsync(counters, 0, attempt == 0 ? 40 : 16, stream);
         fillk::SweepArgs a;
         a.verbs = batch->verbs;
         a.points = batch->points;
@@ -335,7 +439,6 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
         a.num_options = num_options;
         a.order = order;
         a.num_items = items;
-        a.lanes = lanes;
         a.counters = counters;
         a.stage_tops = tops;
         a.heaps = reinterpret_cast<uint32_t*>(fb.scratch);
@@ -355,56 +458,67 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
         a.stage_sfirst = reinterpret_cast<uint32_t*>(fb.stage_sfirst);
         a.stage_s_cap = fb.stage_s_cap / 12;
         a.stage_soff = reinterpret_cast<unsigned long long*>(fb.stage_soff);
+        const uint32_t blocks = std::min(nthreads, items);
+        const bool by_threads = tiny && attempt == 0 && order;
+        a.lanes = lanes;
+        a.size_counters = by_threads ? size_counters : nullptr;
+        a.thread_heap_words =
+            (uint32_t)(heap_bytes / 4 / ((size_t)nthreads * a.lanes)) & ~3u;
         if (sources) {
-            fillk::fill_sweep_kernel<true><<<nthreads, 32, 0, stream>>>(a);
+            fillk::fill_warp_kernel<true><<<blocks, 32, 0, stream>>>(a);
+            if (by_threads) fillk::fill_sweep_kernel<true><<<nthreads, 32, 0, stream>>>(a);
         } else {
-            fillk::fill_sweep_kernel<false><<<nthreads, 32, 0, stream>>>(a);
+            fillk::fill_warp_kernel<false><<<blocks, 32, 0, stream>>>(a);
+            if (by_threads) fillk::fill_sweep_kernel<false><<<nthreads, 32, 0, stream>>>(a);
         }
+        if (by_threads) lg::note_launches(1);
         lg::note_launches(1);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             if (error) *error = std::string("fill sweep: ") + cudaGetErrorString(e);
             return LYON_ERR_CUDA;
         }
-        uint32_t h_ctl[3];
-        unsigned long long h_tops[3];
-        cudaMemcpyAsync(h_ctl, counters, 12, cudaMemcpyDeviceToHost, stream);
-        cudaMemcpyAsync(h_tops, tops, 24, cudaMemcpyDeviceToHost, stream);
+        struct {
+            uint32_t ctl[4];
+            unsigned long long tops[3];
+        } h;
+        static_assert(sizeof(h) == 40, "the counters and, behind them, the staging tops");
+        cudaMemcpyAsync(&h, counters, sizeof(h), cudaMemcpyDeviceToHost, stream);
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
             if (error) *error = std::string("fill sweep: ") + cudaGetErrorString(e);
             return LYON_ERR_CUDA;
         }
-        if (h_ctl[1] == 0) break;
+        if (h.ctl[1] == 0) break;
         // Some paths ran out of heap or staging room: more of both, then only those paths.
         // The staging tops stay where they are (the failed reservations are abandoned).
         const bool staging_short =
-            h_tops[0] > fb.stage_v_cap / 8 || h_tops[1] > fb.stage_i_cap / 4;
-        if (sources && h_tops[2] > fb.stage_s_cap / 12) {
-            const size_t used_s = std::min<size_t>(h_tops[2], fb.stage_s_cap / 12);
-            if (!grow(&fb.stage_s, &fb.stage_s_cap, (size_t)h_tops[2] * 2 * 12 + 4096,
+            h.tops[0] > fb.stage_v_cap / 8 || h.tops[1] > fb.stage_i_cap / 4;
+        if (sources && h.tops[2] > fb.stage_s_cap / 12) {
+            const size_t used_s = std::min<size_t>(h.tops[2], fb.stage_s_cap / 12);
+            if (!grow(&fb.stage_s, &fb.stage_s_cap, (size_t)h.tops[2] * 2 * 12 + 4096,
                       used_s * 12, stream, fb.pool)) {
                 if (error) *error = "cudaMalloc (fill source staging)";
                 return LYON_ERR_OUT_OF_MEMORY;
             }
         }
         if (staging_short) {
-            const size_t used_v = std::min<size_t>(h_tops[0], fb.stage_v_cap / 8);
-            const size_t used_i = std::min<size_t>(h_tops[1], fb.stage_i_cap / 4);
-            if (!grow(&fb.stage_v, &fb.stage_v_cap, (size_t)h_tops[0] * 2 * 8 + 4096,
+            const size_t used_v = std::min<size_t>(h.tops[0], fb.stage_v_cap / 8);
+            const size_t used_i = std::min<size_t>(h.tops[1], fb.stage_i_cap / 4);
+            if (!grow(&fb.stage_v, &fb.stage_v_cap, (size_t)h.tops[0] * 2 * 8 + 4096,
                       used_v * 8, stream, fb.pool) ||
-                !grow(&fb.stage_i, &fb.stage_i_cap, (size_t)h_tops[1] * 2 * 4 + 4096,
+                !grow(&fb.stage_i, &fb.stage_i_cap, (size_t)h.tops[1] * 2 * 4 + 4096,
                       used_i * 4, stream, fb.pool) ||
                 (sources && !grow(&fb.stage_sfirst, &fb.stage_sfirst_cap,
-                                  (size_t)h_tops[0] * 2 * 4 + 4096, used_v * 4, stream,
+                                  (size_t)h.tops[0] * 2 * 4 + 4096, used_v * 4, stream,
                                   fb.pool))) {
                 if (error) *error = "cudaMalloc (fill staging)";
                 return LYON_ERR_OUT_OF_MEMORY;
             }
         }
-        if (h_ctl[2] > 0) fb.heap_words *= 4;
+        if (h.ctl[2] > 0) fb.heap_words *= 4;
         order = lists[attempt & 1];
-        items = h_ctl[1];
+        items = h.ctl[1];
     }
     (void)small_words;
     return LYON_OK;

@@ -11,7 +11,7 @@ namespace lg {
 
 // Device buffers the fill pipeline keeps between its count and emit phases.
 struct FillBuffers {
-    void* scratch = nullptr;        // per-thread sweep heaps
+    void* scratch = nullptr;        // sweep heaps, one per warp
     size_t scratch_cap = 0;
     void* stage_v = nullptr;        // staged vertices (f32 x2) per path
     size_t stage_v_cap = 0;
@@ -21,11 +21,12 @@ struct FillBuffers {
     size_t stage_off_cap = 0;
     void* work = nullptr;           // counters, staging tops and retry lists
     size_t work_cap = 0;
-    uint32_t heap_words = 0;        // per-thread sweep heap size (grows when a path needs more)
+    uint32_t heap_words = 0;        // a warp's heap (grows when a path needs more)
     // Most sweep blocks per SM (0: the default, FILL_SWEEPERS_PER_SM). The serving loop lowers
     // it so that stroke kernels launched meanwhile find room on every SM.
     uint32_t blocks_per_sm_cap = 0;
-    // Sweepers per one-warp block (1..32); 0: chosen per launch from its paths per block.
+    // Threads of a one-warp block that sweep tiny paths (1..32); 0: chosen per launch from its paths
+    // per block.
     uint32_t lanes = 0;
     // When set, every buffer here comes from this pool in stream order (serving contexts).
     cudaMemPool_t pool = nullptr;

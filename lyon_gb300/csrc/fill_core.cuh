@@ -1,11 +1,11 @@
 // fill_core.cuh — lyon's FillTessellator (crates/tessellation/src/fill.rs, event_queue.rs,
-// monotone.rs) as device code run by one thread per path.
+// monotone.rs): the arithmetic that both sweeps share (fill_warp.cuh, a warp per path;
+// fill_sweep.cuh, a thread per path), and the structures of the thread's.
 //
-// The sweep line is sequential within a path, so a thread owns a path from event-queue
-// construction to the last span flush. Its growable arrays (events, active edges, spans and
-// each span's monotone tessellator state) live in a private bump-allocated heap in device
-// memory; a heap that runs out marks the path (FILL_ERR_HEAP) and the host re-runs such paths
-// with larger heaps. Every arithmetic step follows lyon's order of operations in f32 (f64 where
+// A warp or a thread owns a path from event-queue construction to the last span flush. Its growable
+// arrays (events, active edges, spans) live in a private bump-allocated heap in device memory; a
+// heap that runs out marks the path (FILL_ERR_HEAP) and the host re-runs such paths by warps, with
+// larger heaps. Every arithmetic step follows lyon's order of operations in f32 (f64 where
 // lyon uses f64: segment intersections), so outputs match the CPU implementation bit for bit.
 #pragma once
 

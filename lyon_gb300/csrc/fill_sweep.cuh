@@ -1,6 +1,6 @@
-// fill_sweep.cuh — the per-path sweep of the fill tessellator (see fill.cu for the batching).
-// The Filler runs one path from event-queue construction to the last span flush; it compiles for
-// the device (one thread per path) and, for tests and profiling, for the host.
+// fill_sweep.cuh — the fill tessellator's sweep of one path by one thread: the tiny paths of large
+// batches (fill.cu has the rule, fill_warp.cuh the sweep of all others). The Filler runs one path
+// from event-queue construction to the last span flush.
 #pragma once
 
 #include "fill_core.cuh"
