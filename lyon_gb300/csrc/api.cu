@@ -269,6 +269,7 @@ struct VerbCount {
     int grid;
     uint32_t words[lg::STROKE_VERBS_READ];
     bool retry;
+    bool finished;  // the counting launch has done the limit, the scan and the totals
 };
 bool finish_counts(lyon_gpu_context* ctx, uint32_t n, int index_bits, int index_mode,
                    uint64_t vertex_offset, uint64_t* tv, uint64_t* ti, uint32_t* failed,
@@ -276,18 +277,20 @@ bool finish_counts(lyon_gpu_context* ctx, uint32_t n, int index_bits, int index_
     cudaStream_t s = ctx->stream;
     uint32_t* sw = small_words(ctx);
     uint64_t maxi = max_index_for(index_bits);
-    bool to_walk = verbs != nullptr;
+    bool to_walk = verbs != nullptr, finished = verbs && verbs->finished;
 again:
-    cudaMemsetAsync(sw + 2, 0, 8, s);
+    if (!finished) cudaMemsetAsync(sw + 2, 0, 8, s);
     // Per-path mode applies the index range per path; the global mode only counts failures.
-    if (!set_err(ctx, "per-path limit",
+    if (!finished &&
+        !set_err(ctx, "per-path limit",
                  lg::launch_per_path_limit(
                      as<uint32_t>(ctx->vtx_counts), as<uint32_t>(ctx->idx_counts),
                      as<int32_t>(ctx->status), n, vertex_offset,
                      index_mode == LYON_INDEX_PER_PATH ? maxi : ~0ull, sw + 3, s)))
         return false;
     for (int pass = 0; pass < 2; ++pass) {
-        if (!set_err(ctx, "scan",
+        if (!finished &&
+            !set_err(ctx, "scan",
                      lg::launch_scan_pairs(as<uint32_t>(ctx->vtx_counts),
                                            as<uint32_t>(ctx->idx_counts),
                                            as<uint64_t>(ctx->vtx_offsets),
@@ -297,8 +300,10 @@ again:
             return false;
         if (!ensure_host(ctx, ctx->h_small, 64)) return false;
         uint64_t* hs = reinterpret_cast<uint64_t*>(ctx->h_small.ptr);
-        uint64_t* hs_dev = direct_host_pointer<uint64_t>(hs);
-        if (hs_dev) {
+        uint64_t* hs_dev = finished ? nullptr : direct_host_pointer<uint64_t>(hs);
+        if (finished) {
+            finished = false;
+        } else if (hs_dev) {
             lg::launch_read_totals(as<uint64_t>(ctx->vtx_offsets) + n,
                                    as<uint64_t>(ctx->idx_offsets) + n, sw + 2,
                                    verbs ? verbs->arrays->words : nullptr, hs_dev, s);
@@ -505,10 +510,22 @@ int count_by_verb(lyon_gpu_context* ctx, const lyon_path_batch* batch,
         const lg::StrokeArgs a = stroke_args(ctx, batch, options, num_options, index_bits,
                                              index_mode, vertex_offset);
         const uint32_t hint = need ? need : ctx->verb_count > n ? ctx->verb_count : n;
+        lg::StrokeFinish f{};
+        const lg::StrokeFinish* finish = nullptr;
+        if (n <= lg::STROKE_FINISH_PATHS && ensure_host(ctx, ctx->h_small, 64)) {
+            f.host = direct_host_pointer<uint64_t>(ctx->h_small.ptr);
+            f.vtx_offsets = as<uint64_t>(ctx->vtx_offsets);
+            f.idx_offsets = as<uint64_t>(ctx->idx_offsets);
+            f.vertex_offset = vertex_offset;
+            f.max_index = index_mode == LYON_INDEX_PER_PATH ? max_index_for(index_bits) : ~0ull;
+            f.words = small_words(ctx) + 2;
+            if (f.host) finish = &f;
+        }
         if (!set_err(ctx, "stroke count",
-                     lg::launch_stroke_verbs_count(a, v, hint, ctx->num_sms, side_streams(ctx), s)))
+                     lg::launch_stroke_verbs_count(a, v, hint, ctx->num_sms, side_streams(ctx),
+                                                   finish, s)))
             return LYON_ERR_CUDA;
-        VerbCount c{&a, &v, stroke_grid(ctx, n), {}, false};
+        VerbCount c{&a, &v, stroke_grid(ctx, n), {}, false, finish != nullptr};
         mark(ctx, 1);
         if (!finish_counts(ctx, n, index_bits, index_mode, vertex_offset, tv, ti, failed, &c))
             return LYON_ERR_CUDA;

@@ -19,7 +19,8 @@
 //   4. joins_count_kernel (thread per verb) sizes the general join at each verb's end point from
 //      the recorded neighbours, and walks the irregular verbs;
 //   5. tails_kernel (thread per sub-path) sizes caps and closings;
-//   6. verb_scan_kernel turns the verbs' counts into positions, paths_kernel into path counts.
+//   6. verb_scan_kernel turns the verbs' counts into positions, paths_kernel into path counts; for
+//      few paths finish_kernel does what follows the counts, up to the totals, in one launch.
 // Emit phase: runs_kernel writes the runs (lane = flattened point), joins_emit_kernel the general
 // joins and the irregular verbs, tails_kernel the tails.
 //
@@ -29,8 +30,8 @@
 //
 // Measured, whole calls on one GB300, against the warp-per-path walk for every path: 200,000 curve
 // paths (0.47 G vertices) 36.1 -> 8.7 ms, 400,001 map polylines 15.6 -> 1.75 ms, 10,000 curve paths
-// from and to pinned host memory 9.5 -> 3.6 ms, 1,000 paths of 16 segments 287 -> 283 us, one such
-// path from and to host arrays 231 -> 169 us. The walk was bound by the latency of one warp's
+// from and to pinned host memory 9.5 -> 3.6 ms, 1,000 paths of 16 segments 287 -> 241 us, one such
+// path from and to host arrays 231 -> 157 us. The walk was bound by the latency of one warp's
 // chunks (6,000 to 14,000 cycles for 32 points, its code larger than the instruction cache, the
 // longest path last); here no kernel holds more than one stage's code, and parallelism is in verbs
 // and points.
@@ -1148,9 +1149,26 @@ __global__ void __launch_bounds__(128) tails_kernel(StrokeArgs A, StrokeVerbs S)
 
 // ---- 6. positions ------------------------------------------------------------------------------
 
+// A verb's vertices and index words. The edge into a verb's first join is added here, from the join
+// of the verb before it.
+__device__ __forceinline__ void verb_counts(const StrokeArgs& A, const StrokeVerbs& S, uint32_t v,
+                                            uint32_t nv, uint32_t& a, uint32_t& b) {
+    a = b = 0;
+    const int kind = v < nv ? (int)(S.kind[v] & KIND_MASK) : KIND_NONE;
+    if ((is_segment(kind) || is_end(kind)) && !S.path_walk[S.path[v]]) {
+        a = S.vpre[v];
+        b = S.ipre[v];
+        if (!A.widths && is_segment(kind) && (S.kind[v - 1] & KIND_MASK) != LYON_VERB_BEGIN) {
+            const uint32_t f = S.flags[v];
+            if (flags_nk(f) >= 2 || is_segment(S.kind[v + 1] & KIND_MASK))
+                b += 3u * edge_count_flags(pj_from(S.join[v - 1]),
+                                           f & VF_TOFIRST ? EF_SELF_EQ : 0u);
+        }
+    }
+}
+
 // Exclusive sums of the verbs' counts over the whole batch, in place (modulo 2^32: a position
-// within a path is a difference of two): single-pass scan with decoupled look-back. The edge into
-// a verb's first join is added here, from the join of the verb before it.
+// within a path is a difference of two): single-pass scan with decoupled look-back.
 __global__ void __launch_bounds__(SCAN_THREADS) verb_scan_kernel(StrokeArgs A, StrokeVerbs S) {
     __shared__ uint32_t tile_s;
     __shared__ unsigned long long prefix_s[2];
@@ -1168,20 +1186,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) verb_scan_kernel(StrokeArgs A, S
         unsigned long long sa = 0, sb = 0;
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; ++i) {
-            const uint32_t v = base + i;
-            uint32_t a = 0, b = 0;
-            const int kind = v < nv ? (int)(S.kind[v] & KIND_MASK) : KIND_NONE;
-            if ((is_segment(kind) || is_end(kind)) && !S.path_walk[S.path[v]]) {
-                a = S.vpre[v];
-                b = S.ipre[v];
-                if (!A.widths && is_segment(kind) &&
-                    (S.kind[v - 1] & KIND_MASK) != LYON_VERB_BEGIN) {
-                    const uint32_t f = S.flags[v];
-                    if (flags_nk(f) >= 2 || is_segment(S.kind[v + 1] & KIND_MASK))
-                        b += 3u * edge_count_flags(pj_from(S.join[v - 1]),
-                                                   f & VF_TOFIRST ? EF_SELF_EQ : 0u);
-                }
-            }
+            uint32_t a, b;
+            verb_counts(A, S, base + i, nv, a, b);
             va[i] = a;
             vb[i] = b;
             sa += a;
@@ -1231,6 +1237,103 @@ __global__ void __launch_bounds__(256) paths_kernel(StrokeArgs A, StrokeVerbs S)
         A.vtx_counts[path] = vc;
         A.idx_counts[path] = ic;
         A.status[path] = LYON_OK;
+    }
+}
+
+// All that follows the verbs' counts, by one block: with VERBS their positions, then the paths'
+// counts (paths_kernel), the index range per path, the paths' places and the totals (the kernels of
+// scan.cu). For few paths these are short kernels one after another, of which the launches are most:
+// five, with three fills of words before them, for which one path's call took 169 us and takes 157, and
+// 1,000 paths of 16 segments 267 and 241.
+template <bool VERBS>
+__global__ void __launch_bounds__(SCAN_THREADS) finish_kernel(StrokeArgs A, StrokeVerbs S,
+                                                              StrokeFinish F) {
+    __shared__ uint32_t failed_s;
+    const uint32_t v0 = A.verb_offsets[0], nv = batch_verbs(A);
+    if (threadIdx.x == 0) failed_s = 0;
+    __syncthreads();
+    if (VERBS && nv <= S.cap) {
+        unsigned long long pa = 0, pb = 0;
+        for (uint32_t at = 0; at < nv; at += SCAN_TILE) {
+            const uint32_t base = at + threadIdx.x * SCAN_ITEMS;
+            uint32_t va[SCAN_ITEMS], vb[SCAN_ITEMS];
+            unsigned long long sa = 0, sb = 0;
+#pragma unroll
+            for (int i = 0; i < SCAN_ITEMS; ++i) {
+                verb_counts(A, S, base + i, nv, va[i], vb[i]);
+                sa += va[i];
+                sb += vb[i];
+            }
+            unsigned long long ta, tb;
+            const unsigned long long ea = block_excl_scan(sa, &ta), eb = block_excl_scan(sb, &tb);
+            uint32_t ra = (uint32_t)(pa + ea), rb = (uint32_t)(pb + eb);
+#pragma unroll
+            for (int i = 0; i < SCAN_ITEMS; ++i) {
+                if (base + i < nv) {
+                    S.vpre[base + i] = ra;
+                    S.ipre[base + i] = rb;
+                }
+                ra += va[i];
+                rb += vb[i];
+            }
+            pa += ta;
+            pb += tb;
+        }
+        if (threadIdx.x == 0 && nv > 0) {
+            S.vpre[nv] = (uint32_t)pa;
+            S.ipre[nv] = (uint32_t)pb;
+        }
+        __syncthreads();
+    }
+    const bool unfit = nv > S.cap || S.words[1] != 0;
+    unsigned long long pa = 0, pb = 0;
+    for (uint32_t at = 0; at < A.num_paths; at += SCAN_THREADS) {
+        const uint32_t path = at + threadIdx.x;
+        uint32_t vc = 0, ic = 0;
+        if (path < A.num_paths) {
+            int32_t status = LYON_OK;
+            if (!unfit) {
+                const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
+                if (nv > 0) {
+                    const uint32_t pv = S.vpre[s0], pi = S.ipre[s0];
+                    vc = S.vpre[s1] - pv;
+                    ic = S.ipre[s1] - pi;
+                    S.path_v[path] = pv;
+                    S.path_i[path] = pi;
+                }
+                if (S.path_walk[path]) S.walk_list[atomicAdd(&S.words[2], 1u)] = path;
+            }
+            if (vc > 0 && F.vertex_offset + vc - 1 > F.max_index) {
+                status = LYON_ERR_TOO_MANY_VERTICES;
+                vc = ic = 0;
+                atomicAdd(&failed_s, 1u);
+            }
+            A.vtx_counts[path] = vc;
+            A.idx_counts[path] = ic;
+            A.status[path] = status;
+        }
+        unsigned long long ta, tb;
+        const unsigned long long ea = block_excl_scan((unsigned long long)vc, &ta);
+        const unsigned long long eb = block_excl_scan((unsigned long long)ic, &tb);
+        if (path < A.num_paths) {
+            F.vtx_offsets[path] = pa + ea;
+            F.idx_offsets[path] = pb + eb;
+        }
+        pa += ta;
+        pb += tb;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        F.vtx_offsets[A.num_paths] = pa;
+        F.idx_offsets[A.num_paths] = pb;
+        F.words[0] = 0;
+        F.words[1] = failed_s;
+        F.host[0] = pa;
+        F.host[1] = pb;
+        F.host[2] = (uint64_t)failed_s << 32;
+        const volatile uint32_t* w = S.words;
+        F.host[3] = (uint64_t)w[0] | ((uint64_t)w[1] << 32);
+        F.host[4] = (uint64_t)w[2] | ((uint64_t)w[3] << 32);
     }
 }
 
@@ -1504,7 +1607,7 @@ uint32_t grid_for(uint32_t items, uint32_t per_block, int num_sms, uint32_t wave
 
 cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
                                       uint32_t verbs_hint, int num_sms, const SideStreams& side,
-                                      cudaStream_t s) {
+                                      const StrokeFinish* finish, cudaStream_t s) {
     const uint32_t n = a.num_paths;
     cudaMemsetAsync(v.words, 0, v.clear_bytes, s);
     const uint32_t by_path = grid_for(n, 8, num_sms, 8);
@@ -1525,9 +1628,20 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
         side.join(0, s);
         note_launches(3);
     }
+    note_launches(5);
+    // One tile of verbs is summed by the block that finishes; more by as many blocks.
+    const bool one_tile = finish && verbs_hint <= SCAN_TILE;
+    if (one_tile) {
+        finish_kernel<true><<<1, SCAN_THREADS, 0, s>>>(a, v, *finish);
+        return cudaGetLastError();
+    }
     verb_scan_kernel<<<grid_for(verbs_hint, SCAN_TILE, num_sms, 4), SCAN_THREADS, 0, s>>>(a, v);
-    paths_kernel<<<grid_for(n, 256, num_sms, 8), 256, 0, s>>>(a, v);
-    note_launches(6);
+    if (finish) {
+        finish_kernel<false><<<1, SCAN_THREADS, 0, s>>>(a, v, *finish);
+    } else {
+        paths_kernel<<<grid_for(n, 256, num_sms, 8), 256, 0, s>>>(a, v);
+    }
+    note_launches(1);
     return cudaGetLastError();
 }
 
@@ -1544,8 +1658,10 @@ cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
             a, v);
         note_launches(1);
     }
+    // (joins and tails are the shorter ones of a small batch, and share a stream: 1,000 paths of 16
+    // segments take 12 and 47 us there, the runs 59, the verbs apart 77)
     extra_emit_kernel<<<grid_for(verbs_hint / 8, 128, num_sms, 8), 128, 0, j>>>(a, v);
-    joins_emit_kernel<<<grid_for(verbs_hint, 256, num_sms, 8), 256, 0, j>>>(a, v);
+    joins_emit_kernel<<<grid_for(verbs_hint, 256, num_sms, 8), 256, 0, t>>>(a, v);
     tails_kernel<true><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
     note_launches(3);
     side.join(0, s);

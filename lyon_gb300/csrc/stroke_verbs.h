@@ -62,11 +62,21 @@ struct SideStreams {
     }
 };
 
+// What follows the counts of a batch of few paths, in the same launch: the index range per path, the
+// paths' places, and the totals.
+constexpr uint32_t STROKE_FINISH_PATHS = 2048;
+struct StrokeFinish {
+    uint64_t *vtx_offsets, *idx_offsets;
+    uint64_t vertex_offset, max_index;  // max_index: per path, ~0 for none
+    uint32_t* words;                    // [0] scan error, [1] failed paths
+    uint64_t* host;                     // totals, the words above, STROKE_VERBS_READ words
+};
 // Counts of every path (vtx_counts, idx_counts, status of `a`), the paths in walk_list apart.
-// `verbs_hint`: about how many verbs the batch has (sizes the grids only).
+// `verbs_hint`: about how many verbs the batch has (sizes the grids, and with `finish`, which may be
+// null, chooses who sums the verbs). finish: for STROKE_FINISH_PATHS paths at most.
 cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
                                       uint32_t verbs_hint, int num_sms, const SideStreams& side,
-                                      cudaStream_t s);
+                                      const StrokeFinish* finish, cudaStream_t s);
 // The stepper's part of it (stroke_steps.cu): counts of a variable-width stroke once the kept points
 // are known, and the output of variable widths, vertex sources and attribute records.
 void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint,

@@ -314,3 +314,17 @@ def test_stepped_small_batches(ctx, n):
         o = options(np.random.default_rng(n), 1, tol=0.05)
         o["line_width"] = 3.0
         same_bits(stepped(ctx, batch, o, how, by_path=True), stepped(ctx, batch, o, how))
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 2047, 2048, 2049])
+def test_counts_finished_by_one_block(ctx, n):
+    # Up to 2,048 paths one block sums paths and, for a tile of 2,048 verbs or fewer as the call
+    # before had, the verbs; the batch here has more verbs than that call. At this vertex offset
+    # the longer paths pass the range of 16-bit indices and fail.
+    rng = np.random.default_rng(n)
+    first = rough_paths(3, n)
+    check(ctx, first, options(rng, first.num_paths))
+    batch = rough_paths(n, n + 1, 12)
+    opts = options(rng, batch.num_paths)
+    check(ctx, batch, opts)
+    check(ctx, batch, opts, 16, T.INDEX_PER_PATH, 65500)
