@@ -17,9 +17,9 @@
 //
 // Bound by instruction issue with 9 to 12 of a warp's 32 lanes at work (curves of different lengths,
 // general joins among flattening steps). Measured, whole calls on one GB300, against one thread
-// per path (records: one warp): variable width on 10,001 curve paths 159 -> 7.1 ms, vertex
-// sources and two custom values on 9,999 paths 82 -> 2.3 ms, records on 20,000 paths 6.3 -> 5.2 ms
-// (of which the advancement 1.7).
+// per path (records: one warp): variable width on 10,001 curve paths 159 -> 7.0 ms, vertex
+// sources and two custom values on 9,999 paths 82 -> 2.3 ms, records on 20,000 paths 6.3 -> 4.6 ms
+// (of which the advancement 1.0).
 #include "stroke_seq.cuh"
 #include "stroke_verbs.cuh"
 
@@ -613,17 +613,22 @@ uint32_t blocks_for(uint32_t items, uint32_t per_block, int num_sms, uint32_t wa
     return need < sms ? sms : need > sms * waves ? sms * waves : need;
 }
 
-void launch_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms, cudaStream_t s) {
-    advance_long_kernel<<<blocks_for(a.num_paths, 1, num_sms, 8), 256, 0, s>>>(a, v);
+// Side by side: the long paths are few blocks, each bound by its chain of additions (20,000 records
+// paths: 0.93 and 0.76 ms one after the other).
+void launch_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
+                    const SideStreams& side, cudaStream_t s) {
+    const cudaStream_t l = side.fork(0, s);
+    advance_long_kernel<<<blocks_for(a.num_paths, 1, num_sms, 8), 256, 0, l>>>(a, v);
     advance_kernel<<<blocks_for(a.num_paths, 4, num_sms, 16), 128, 0, s>>>(a, v);
+    side.join(0, s);
     note_launches(2);
 }
 
 }  // namespace
 
 void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint,
-                               int num_sms, cudaStream_t s) {
-    launch_advance(a, v, num_sms, s);
+                               int num_sms, const SideStreams& side, cudaStream_t s) {
+    launch_advance(a, v, num_sms, side, s);
     steps_kernel<false, true, Sink>
         <<<blocks_for(verbs_hint, STEP_TILE, num_sms, 16), 128, 0, s>>>(a, v);
     check_states_kernel<<<blocks_for(verbs_hint, 256, num_sms, 8), 256, 0, s>>>(a, v);
@@ -631,7 +636,8 @@ void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32
 }
 
 cudaError_t launch_stroke_steps_emit(const StrokeArgs& a, const StrokeVerbs& v,
-                                     uint32_t verbs_hint, int num_sms, cudaStream_t s) {
+                                     uint32_t verbs_hint, int num_sms, const SideStreams& side,
+                                     cudaStream_t s) {
     const uint32_t grid = blocks_for(verbs_hint, STEP_TILE, num_sms, 16);
     if (a.widths) {
         if (a.sources && a.vertex_attrs) {
@@ -645,7 +651,7 @@ cudaError_t launch_stroke_steps_emit(const StrokeArgs& a, const StrokeVerbs& v,
         }
     } else {
         if (a.vertex_attrs) {
-            launch_advance(a, v, num_sms, s);
+            launch_advance(a, v, num_sms, side, s);
         }
         if (a.sources && a.vertex_attrs) {
             steps_kernel<true, false, SrcSinkT<true>><<<grid, 128, 0, s>>>(a, v);

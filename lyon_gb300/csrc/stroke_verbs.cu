@@ -1618,7 +1618,7 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
                   WIN_WARPS * sizeof(WalkSmem), s>>>(a, v);
     drops_kernel<<<grid_for(0, 128, num_sms, 1), 128, 0, s>>>(a, v);
     if (a.widths) {
-        launch_stroke_steps_count(a, v, verbs_hint, num_sms, s);
+        launch_stroke_steps_count(a, v, verbs_hint, num_sms, side, s);
     } else {
         // Tails read the points beside the sub-paths' ends and nothing of the joins.
         const cudaStream_t t = side.fork(0, s);
@@ -1649,7 +1649,7 @@ cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
                                      uint32_t verbs_hint, bool runs, int num_sms,
                                      const SideStreams& side, cudaStream_t s) {
     if (a.widths || a.sources || a.vertex_attrs)
-        return launch_stroke_steps_emit(a, v, verbs_hint, num_sms, s);
+        return launch_stroke_steps_emit(a, v, verbs_hint, num_sms, side, s);
     // The three write different parts of the output; joins and tails are short of warps and of
     // threads that agree, and fill the gaps of the runs.
     const cudaStream_t j = side.fork(0, s), t = side.fork(1, s);

@@ -80,9 +80,10 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
 // The stepper's part of it (stroke_steps.cu): counts of a variable-width stroke once the kept points
 // are known, and the output of variable widths, vertex sources and attribute records.
 void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint,
-                               int num_sms, cudaStream_t s);
+                               int num_sms, const SideStreams& side, cudaStream_t s);
 cudaError_t launch_stroke_steps_emit(const StrokeArgs& a, const StrokeVerbs& v,
-                                     uint32_t verbs_hint, int num_sms, cudaStream_t s);
+                                     uint32_t verbs_hint, int num_sms, const SideStreams& side,
+                                     cudaStream_t s);
 // Output of the paths that launch_stroke_verbs_count counted. `runs`: words[3].
 cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
                                      uint32_t verbs_hint, bool runs, int num_sms,
