@@ -17,6 +17,7 @@ struct FillBuffers {
     size_t stage_v_cap = 0;
     void* stage_i = nullptr;        // staged indices (u32, path-relative) per path
     size_t stage_i_cap = 0;
+    uint32_t stage_paths = 0;       // most paths of a batch the staging was sized for
     void* stage_off = nullptr;      // per path: staged vertex/index base (u64 x2)
     size_t stage_off_cap = 0;
     void* work = nullptr;           // counters, staging tops and retry lists
