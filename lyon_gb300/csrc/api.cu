@@ -431,6 +431,7 @@ lg::StrokeVerbs stroke_verbs(lyon_gpu_context* ctx, uint32_t n) {
     v.cap = ctx->verb_cap - 1;
     v.firsts = reinterpret_cast<float4*>(take(cap * 16));
     v.lasts = reinterpret_cast<float4*>(take(cap * 16));
+    v.adv = reinterpret_cast<float4*>(take(cap * 16));
     v.fin = reinterpret_cast<float2*>(take(cap * 8));
     v.rec = reinterpret_cast<uint32_t*>(take(cap * 4));
     v.path = reinterpret_cast<uint32_t*>(take(cap * 4));
@@ -621,12 +622,7 @@ int pipeline_emit(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch,
                                        num_options, index_bits, index_mode, vertex_offset);
         a.vertices = vout;
         a.indices = iout;
-        // Records of a small batch are written by the walk of a warp per path: the verbs' steppers
-        // take 1.5 ms to a verb's end however few there are (300 curve paths, 6,000 verbs: 0.93 ms
-        // by path, 1.50 by verb; 3,000 paths: 2.56 and 1.92).
-        const bool small_records = ctx->vertex_attrs && !ctx->want_sources && !ctx->vw_widths &&
-                                   ctx->verb_count < 32768u;
-        if (n > 0 && tv > 0 && ctx->verbs_valid && !small_records) {
+        if (n > 0 && tv > 0 && ctx->verbs_valid) {
             const lg::StrokeVerbs v = stroke_verbs(ctx, n);
             if (!set_err(ctx, "stroke emit",
                          lg::launch_stroke_verbs_emit(a, v, ctx->verb_count, ctx->verb_runs,

@@ -17,12 +17,12 @@
 // The active edges, pending edges and span list of a path are in shared memory as long as they
 // fit (longer ones move to the heap).
 //
-// What bounds it: the dependent instructions of one event after another in small launches (about
-// 700 instructions and 4,500 cycles per event, alone on an SM), instruction fetch in large ones:
-// with 16 warps on an SM, each at another place of the code, a warp waits for its next instruction
-// 60 % of the time, so the code is kept small (rare steps out of line, loops not unrolled: 250 to
-// 143 KB made 30,000 glyph paths 1.5 times faster). Times, a thread per path and a warp per path: one
-// glyph of 1,083 events 11.6 and 3.0 ms, 777 glyphs 47.8 and 9.9 ms, 30,000 glyphs 361 and 54 ms.
+// What bounds it: the dependent instructions of one event after another (about 700 instructions, 7
+// cycles each with four warps on an SM; 40 % of that is fixed latency). Code size comes next: with 16
+// warps on an SM, each at another place of 250 KB of code, a warp waited for its next instruction
+// 60 % of the time, so rare steps are out of line and loops are not unrolled (143 KB: 30,000 glyph
+// paths 1.5 times faster). Times, a thread per path and a warp per path: one glyph of 1,083 events
+// 11.6 and 3.0 ms, 777 glyphs 47.8 and 9.9 ms, 30,000 glyphs 361 and 54 ms.
 // Warps per SM, for one glyph / 777 / 30,000: 8 (154 registers) 2.8 / 9.6 / 68 ms, 12 2.9 / 9.6 / 59,
 // 16 (128 registers) 3.0 / 10.0 / 55, 20 3.1 / 10.4 / 53, 24 3.3 / 10.6 / 54, 32 3.8 / 11.3 / 58.
 #pragma once

@@ -38,7 +38,7 @@ struct StrokeArgs {
     // side) instead of positions.
     int vertex_attrs;
     // Non-null: variable line width, one width factor per point of the batch (indexed like
-    // `points`); the paths are stroked by the variable-width kernel (one thread per path).
+    // `points`); the paths are stroked by lyon's variable-width stepper.
     const float* widths;
     // Optional, per path: the first path of the request it belongs to. In LYON_INDEX_GLOBAL mode
     // ids then count from that path's first vertex (one VertexBuffers per request of a batch).
@@ -50,8 +50,8 @@ struct StrokeArgs {
     uint32_t* seq_counter;
     // Non-zero: only items [0, *item_split) of the order are stroked.
     int list_only;
-    // Non-zero: every path is stroked by lyon's sequential stepper, one path per thread, in both
-    // passes (set by the custom-attribute calls; `widths` implies it). With `sources` the emit
+    // Non-zero: every path is stroked by lyon's sequential stepper in both passes (set by the
+    // custom-attribute calls; `widths` implies it). With `sources` the emit
     // pass writes each vertex's lyon_vertex_source next to it.
     int sequential;
     lyon_vertex_source* sources;

@@ -8,8 +8,8 @@
 // meanwhile, so their work overlaps on the device. Outputs stay resident in device slabs until
 // the caller releases the request; slabs are pooled per worker and reused.
 //
-// Stroke requests take microseconds to milliseconds of GPU time, fill requests tens of
-// milliseconds (one path's sweep runs on one thread). With stroke workers configured, the kinds
+// Stroke requests take microseconds to milliseconds of GPU time, fill requests about ten
+// milliseconds (one path's sweep runs on one warp). With stroke workers configured, the kinds
 // get separate workers: stroke workers run on streams of the device's highest priority with one
 // stroke block per SM, and fill sweeps keep at most `fill_blocks_per_sm` blocks per SM, so that
 // a stroke launch finds room on every SM and starts while fill sweeps are running instead of

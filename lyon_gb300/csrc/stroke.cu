@@ -1,4 +1,6 @@
-// stroke.cu — batched fixed-width stroke tessellation (count and emit kernels).
+// stroke.cu — batched fixed-width stroke tessellation, a path as a whole (count and emit kernels): the
+// paths that the verb-parallel stroke (stroke_verbs.cu) leaves, batches it cannot take and the
+// no-allocation entry.
 //
 // One warp strokes one path at a time; warps of a persistent grid take paths from an atomic
 // work counter. lyon's stroker (stroke.rs:1521-1632) is a sequential state machine over the

@@ -1,6 +1,6 @@
 // stroke_steps.cu — lyon's sequential stroke stepper, one verb per thread.
 //
-// Variable line width, vertex sources and attribute records want the stepper itself
+// Variable line width and vertex sources want the stepper itself
 // (stroke_seq.cuh, stroke_core.cuh). Its state is short: the last two points with their sides,
 // ids and advancement. So a thread can step one verb by itself once it has that state, which it
 // gets by stepping the last four kept points before the verb first, without output (a point's
@@ -15,11 +15,12 @@
 // thread as a whole (stroke_seq.cu), as are the paths that stroke_verbs.cu leaves out. (A clipped
 // miter moves side points of the joins after it, so those paths usually go that way.)
 //
+// The advancement kernels also serve attribute records, which stroke_verbs.cu writes run by run.
+//
 // Bound by instruction issue with 9 to 12 of a warp's 32 lanes at work (curves of different lengths,
 // general joins among flattening steps). Measured, whole calls on one GB300, against one thread
-// per path (records: one warp): variable width on 10,001 curve paths 159 -> 7.0 ms, vertex
-// sources and two custom values on 9,999 paths 82 -> 2.3 ms, records on 20,000 paths 6.3 -> 4.6 ms
-// (of which the advancement 1.0).
+// per path: variable width on 10,001 curve paths 159 -> 6.9 ms, vertex sources and two custom values
+// on 9,999 paths 82 -> 2.3 ms.
 #include "stroke_seq.cuh"
 #include "stroke_verbs.cuh"
 
@@ -27,7 +28,7 @@ namespace lg {
 namespace {
 
 // The four advancements kept per verb: those of its last four kept points (.w: the last one).
-__device__ __forceinline__ float4* advancements(const StrokeVerbs& S) { return S.firsts; }
+__device__ __forceinline__ float4* advancements(const StrokeVerbs& S) { return S.adv; }
 __device__ __forceinline__ float advancement_back(const StrokeVerbs& S, uint32_t v, uint32_t back) {
     return reinterpret_cast<const float*>(advancements(S) + v)[3u - back];
 }
@@ -63,6 +64,7 @@ __device__ __forceinline__ void advance_special(const StrokeArgs& A, const Strok
         verb_units(kind, S.rec[v], A.points, P.tolerance, flags & VF_TURN,
                    flags & VF_TURN ? S.cut[v] : 0u, a, b);
         V2 last = last_kept(S, A.points, v - 1);
+        float before = st.adv;  // at the last kept point but one
         for (uint32_t u = 0; u < (b.m ? 2u : 1u); ++u) {
             float t = a.t0;
             for (uint32_t k = 1; k <= a.m; ++k) {
@@ -72,18 +74,23 @@ __device__ __forceinline__ void advance_special(const StrokeArgs& A, const Strok
                     q = poly_sample(a.p, t);
                 }
                 if (too_close(last, q, P.merge_threshold)) continue;
+                before = st.adv;
                 st.adv = st.adv + vlength(q - last);
                 last = q;
                 ++st.kept;
             }
             a = b;
         }
-        if (lane == 0) out[3] = st.adv;
+        if (lane == 0) {
+            out[2] = before;
+            out[3] = st.adv;
+        }
     }
 }
 
-// Calls use(i, len) for the verb's edges 32 at a time: lane's edge i (0-based; >= the verb's edges:
-// none) and its length. Returns the number of edges.
+// Calls use(i, count, len, edges, first) for the verb's edges 32 at a time: lane's edge i (0-based;
+// >= the verb's edges: none) and its length, how many edges the verb has and how many of them are
+// its first run's (0: there is one run only). Returns the number of edges.
 template <class F>
 __device__ __forceinline__ uint32_t verb_edges(const StrokeArgs& A, const StrokeVerbs& S,
                                                uint32_t v, int kind, const StrokeParams& P,
@@ -92,7 +99,7 @@ __device__ __forceinline__ uint32_t verb_edges(const StrokeArgs& A, const Stroke
     Unit a, b;
     verb_units(kind, S.rec[v], A.points, P.tolerance, flags, flags & VF_TWO ? S.cut[v] : 0u, a, b);
     V2 last = last_kept(S, A.points, v - 1);
-    const uint32_t M = a.m + b.m;
+    const uint32_t M = a.m + b.m, first = b.m ? a.m : 0u;
     uint32_t before = 0;
     for (uint32_t u = 0; u < (b.m ? 2u : 1u); ++u) {
         uint32_t tk = 0;
@@ -103,7 +110,7 @@ __device__ __forceinline__ uint32_t verb_edges(const StrokeArgs& A, const Stroke
             const V2 q = kk == a.m ? a.to : poly_sample(a.p, t);
             V2 p = V2{__shfl_up_sync(FULL, q.x, 1), __shfl_up_sync(FULL, q.y, 1)};
             if (lane == 0) p = last;
-            use((uint32_t)lane < cnt ? before + kk - 1u : M, cnt, vlength(q - p), M);
+            use((uint32_t)lane < cnt ? before + kk - 1u : M, cnt, vlength(q - p), M, first);
             last = V2{__shfl_sync(FULL, q.x, (int)cnt - 1), __shfl_sync(FULL, q.y, (int)cnt - 1)};
             tk = k0 + cnt - 1u;
             t0 = __shfl_sync(FULL, t, (int)cnt - 1);
@@ -117,6 +124,14 @@ __device__ __forceinline__ uint32_t verb_edges(const StrokeArgs& A, const Stroke
 // Paths of more verbs than this are taken by blocks (below), the others by warps.
 constexpr uint32_t ADVANCE_LONG = 64;
 
+// The advancement at edge e's end, of M, where it is one of the last four; with `first` (the edges of
+// the first of two runs) the one between the runs takes the first place.
+__device__ __forceinline__ void keep_advancement(float* out, uint32_t e, uint32_t M, uint32_t first,
+                                                 float adv) {
+    if (e < M && e + (first ? 3u : 4u) >= M) out[4u - (M - e)] = adv;
+    if (first && e + 1u == first) out[0] = adv;
+}
+
 // Warp per path. Bound by the sum's chain, 32 additions for 32 points.
 __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs S) {
     const int lane = threadIdx.x & 31;
@@ -125,6 +140,7 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
     if (batch_verbs(A) > S.cap || S.words[1] != 0) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
+    const bool runs = !A.widths && !A.sources;  // records: written run by run (stroke_verbs.cu)
     for (uint32_t path = warp; path < A.num_paths; path += nwarps) {
         const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
         if (s1 - s0 > ADVANCE_LONG || S.path_walk[path]) continue;
@@ -141,7 +157,7 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
                     continue;
                 }
                 st.kept += verb_edges(A, S, v, k, P, lane, [&](uint32_t e, uint32_t cnt, float len,
-                                                               uint32_t M) {
+                                                               uint32_t M, uint32_t m1) {
                     float mine = 0.0f;
 #pragma unroll
                     for (uint32_t j = 0; j < 32; ++j) {
@@ -149,7 +165,7 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
                         st.adv = st.adv + (j < cnt ? x : 0.0f);
                         if ((uint32_t)lane == j) mine = st.adv;
                     }
-                    if (e < M && e + 4u >= M) out[4 * (size_t)v + 4u - (M - e)] = mine;
+                    keep_advancement(out + 4 * (size_t)v, e, M, runs ? m1 : 0u, mine);
                 });
             }
         }
@@ -163,12 +179,14 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
     __shared__ float4 room[ADVANCE_ROOM / 4];
     __shared__ uint32_t first[33];
     __shared__ int kinds[32];
+    __shared__ uint32_t split[32];  // edges of the first of two runs, else 0
     __shared__ uint32_t window;
     float* len = reinterpret_cast<float*>(room);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (batch_verbs(A) > S.cap || S.words[1] != 0) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
+    const bool runs = !A.widths && !A.sources;
     for (uint32_t path = blockIdx.x; path < A.num_paths; path += gridDim.x) {
         const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
         if (s1 - s0 <= ADVANCE_LONG || S.path_walk[path]) continue;
@@ -180,7 +198,7 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                 // The window's verbs, their points rounded up to 16-byte words.
                 const uint32_t v = base + (uint32_t)lane;
                 int k = v < s1 ? S.kind[v] & KIND_MASK : KIND_NONE;
-                uint32_t m = 0;
+                uint32_t m = 0, m1 = 0;
                 if (is_segment(k)) {
                     const uint32_t flags = S.flags[v];
                     if (flags & VF_IRR) {
@@ -190,8 +208,10 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                         verb_units(k, S.rec[v], A.points, P.tolerance, flags,
                                    flags & VF_TWO ? S.cut[v] : 0u, a, b);
                         m = a.m + b.m;
+                        if (runs && b.m) m1 = a.m;
                     }
                 }
+                split[lane] = m1;
                 uint32_t incl = (m + 3u) & ~3u;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -209,7 +229,7 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                 const int k = kinds[i] & 15;
                 if (!is_segment(k)) continue;
                 verb_edges(A, S, base + i, k, P, lane,
-                           [&](uint32_t e, uint32_t, float x, uint32_t M) {
+                           [&](uint32_t e, uint32_t, float x, uint32_t M, uint32_t) {
                                if (e < M) len[first[i] + e] = x;
                            });
             }
@@ -218,13 +238,13 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                 // One verb of more points than there is room for.
                 const int k = kinds[0] & 15;
                 st.kept += verb_edges(A, S, base, k, P, lane, [&](uint32_t e, uint32_t cnt, float x,
-                                                                  uint32_t M) {
+                                                                  uint32_t M, uint32_t m1) {
                     float mine = 0.0f;
                     for (uint32_t j = 0; j < cnt; ++j) {
                         st.adv = st.adv + __shfl_sync(FULL, x, (int)j);
                         if ((uint32_t)lane == j) mine = st.adv;
                     }
-                    if (e < M && e + 4u >= M) out[4 * (size_t)base + 4u - (M - e)] = mine;
+                    keep_advancement(out + 4 * (size_t)base, e, M, runs ? m1 : 0u, mine);
                 });
             }
             for (uint32_t i = 0; warp == 0 && i < n; ++i) {
@@ -237,12 +257,16 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                 float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = st.adv;
                 const float4* w = room + first[i] / 4u;
                 uint32_t j = 0;
+                const uint32_t m1 = split[i];
+                float between = 0.0f;
                 for (; j + 4u <= m; j += 4u) {
                     const float4 x = w[j / 4u];
                     a0 = a3 + x.x;
                     a1 = a0 + x.y;
                     a2 = a1 + x.z;
                     a3 = a2 + x.w;
+                    if (m1 > j && m1 <= j + 4u)
+                        between = m1 == j + 1u ? a0 : m1 == j + 2u ? a1 : m1 == j + 3u ? a2 : a3;
                 }
                 for (; j < m; ++j) {
                     const float x = len[first[i] + j];
@@ -250,10 +274,11 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                     a1 = a2;
                     a2 = a3;
                     a3 = a3 + x;
+                    if (m1 == j + 1u) between = a3;
                 }
                 st.adv = a3;
                 st.kept += m;
-                if (lane == 0) advancements(S)[v] = make_float4(a0, a1, a2, a3);
+                if (lane == 0) advancements(S)[v] = make_float4(m1 ? between : a0, a1, a2, a3);
             }
             base += n > 0 ? n : 1u;
         }
@@ -613,10 +638,12 @@ uint32_t blocks_for(uint32_t items, uint32_t per_block, int num_sms, uint32_t wa
     return need < sms ? sms : need > sms * waves ? sms * waves : need;
 }
 
-// Side by side: the long paths are few blocks, each bound by its chain of additions (20,000 records
-// paths: 0.93 and 0.76 ms one after the other).
-void launch_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
-                    const SideStreams& side, cudaStream_t s) {
+}  // namespace
+
+// Side by side: the long paths are few blocks, each bound by its chain of additions (20,000 paths with
+// records: 0.93 and 0.76 ms one after the other).
+void launch_stroke_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
+                           const SideStreams& side, cudaStream_t s) {
     const cudaStream_t l = side.fork(0, s);
     advance_long_kernel<<<blocks_for(a.num_paths, 1, num_sms, 8), 256, 0, l>>>(a, v);
     advance_kernel<<<blocks_for(a.num_paths, 4, num_sms, 16), 128, 0, s>>>(a, v);
@@ -624,11 +651,9 @@ void launch_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
     note_launches(2);
 }
 
-}  // namespace
-
 void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint,
                                int num_sms, const SideStreams& side, cudaStream_t s) {
-    launch_advance(a, v, num_sms, side, s);
+    launch_stroke_advance(a, v, num_sms, side, s);
     steps_kernel<false, true, Sink>
         <<<blocks_for(verbs_hint, STEP_TILE, num_sms, 16), 128, 0, s>>>(a, v);
     check_states_kernel<<<blocks_for(verbs_hint, 256, num_sms, 8), 256, 0, s>>>(a, v);
@@ -651,14 +676,10 @@ cudaError_t launch_stroke_steps_emit(const StrokeArgs& a, const StrokeVerbs& v,
         }
     } else {
         if (a.vertex_attrs) {
-            launch_advance(a, v, num_sms, side, s);
-        }
-        if (a.sources && a.vertex_attrs) {
+            launch_stroke_advance(a, v, num_sms, side, s);
             steps_kernel<true, false, SrcSinkT<true>><<<grid, 128, 0, s>>>(a, v);
-        } else if (a.sources) {
-            steps_kernel<true, false, SrcSinkT<false>><<<grid, 128, 0, s>>>(a, v);
         } else {
-            steps_kernel<true, false, RecSink><<<grid, 128, 0, s>>>(a, v);
+            steps_kernel<true, false, SrcSinkT<false>><<<grid, 128, 0, s>>>(a, v);
         }
     }
     note_launches(1);

@@ -29,7 +29,8 @@
 // the same bit for bit; tests/test_gpu_stroke_verbs.py compares the two.
 //
 // Measured, whole calls on one GB300, against the warp-per-path walk for every path: 200,000 curve
-// paths (0.47 G vertices) 36.1 -> 8.7 ms, 400,001 map polylines 15.6 -> 1.75 ms, 10,000 curve paths
+// paths (0.47 G vertices) 36.1 -> 8.4 ms, 400,001 map polylines 15.6 -> 1.75 ms, attribute records on
+// 20,000 paths 6.4 -> 2.9 ms (by lyon's stepper, a verb per thread, 4.6), 10,000 curve paths
 // from and to pinned host memory 9.5 -> 3.6 ms, 1,000 paths of 16 segments 287 -> 241 us, one such
 // path from and to host arrays 231 -> 157 us. The walk was bound by the latency of one warp's
 // chunks (6,000 to 14,000 cycles for 32 points, its code larger than the instruction cache, the
@@ -712,14 +713,18 @@ struct VerbOut {
     uint32_t pfn, pfp;
     bool edge;            // the next join has an edge into it
     int st;
+    float adv;            // the advancement of the next join (records only)
 };
 
-__device__ __forceinline__ Sink sink_at(const PathOut& po, uint32_t vo, uint32_t io) {
-    Sink s;
+// REC: attribute records instead of positions (here and in the kernels of the emit phase).
+template <bool REC>
+__device__ __forceinline__ SinkT<REC> sink_at(const PathOut& po, uint32_t vo, uint32_t io) {
+    SinkT<REC> s;
     s.id_base = po.id_base + vo;
     s.nv = 0;
     s.ni = 0;
-    s.vout = po.vout + vo;
+    s.vout = REC ? nullptr : po.vout + vo;
+    s.rout = REC ? po.rout + vo : nullptr;
     s.iout = po.bits == 16 ? (void*)((uint16_t*)po.iout + io) : (void*)((uint32_t*)po.iout + io);
     s.index_bits = po.bits;
     s.vcap = cap_left(po.vmax, vo);
@@ -728,10 +733,12 @@ __device__ __forceinline__ Sink sink_at(const PathOut& po, uint32_t vo, uint32_t
     return s;
 }
 
+template <bool REC>
 __device__ __forceinline__ void emit_general(VerbOut& o, V2 prv, V2 cur, bool flat, V2 nxt,
                                              const StrokeParams& P, uint32_t packed) {
-    const JoinEmitOut r = slow_join_emit_at(prv, cur, flat, nxt, P, sink_at(o.po, o.vo, o.io),
-                                            o.edge, o.pfn, o.pfp);
+    SinkT<REC> sk = sink_at<REC>(o.po, o.vo, o.io);
+    if (REC) sk.adv = o.adv;
+    const JoinEmitOut r = slow_join_emit_at(prv, cur, flat, nxt, P, sk, o.edge, o.pfn, o.pfp);
     if (r.st != LYON_OK) o.st = r.st;
     if (r.overflow || r.nv != pj_vertices(packed)) o.st = LYON_ERR_INTERNAL;
     const uint32_t base = o.po.id_base + o.vo;
@@ -743,11 +750,18 @@ __device__ __forceinline__ void emit_general(VerbOut& o, V2 prv, V2 cur, bool fl
 }
 
 // A flattening step's join (stroke.rs:1743-1806) written through `o`.
+template <bool REC>
 __device__ __forceinline__ void emit_step(VerbOut& o, V2 prv, V2 cur, V2 nxt, float hw) {
     const SidePair s = fast_join_sides(prv, cur, nxt, hw);
-    Sink sk = sink_at(o.po, o.vo, o.io);
-    const uint32_t id = sk.vertex(s.pn, V2{0.0f, 0.0f}, SP);
-    sk.vertex(s.nn, V2{0.0f, 0.0f}, SN);
+    SinkT<REC> sk = sink_at<REC>(o.po, o.vo, o.io);
+    V2 n = V2{0.0f, 0.0f};
+    if (REC) {  // (the positions are at n and -n times the half width)
+        const V2 pe = cur - prv, ne = nxt - cur;
+        n = compute_normal(pe / vlength(pe), ne / vlength(ne));
+        sk.adv = o.adv;
+    }
+    const uint32_t id = sk.vertex(s.pn, n, SP);
+    sk.vertex(s.nn, -n, SN);
     if (o.edge) edge_triangles(o.pfn, o.pfp, id + 1, id, &sk);
     if (sk.overflow) o.st = LYON_ERR_INTERNAL;
     o.vo += sk.nv;
@@ -761,7 +775,7 @@ __device__ __forceinline__ void emit_step(VerbOut& o, V2 prv, V2 cur, V2 nxt, fl
 // kept point `c1` before it (the join at c1 belongs to the verb before, the one at the last kept
 // point is not done here). Counts into `sum`, or emits through `o`. Returns false when the path
 // has to be walked as a whole: a join fails, or the skip test is not ruled out by its bound.
-template <bool EMIT>
+template <bool EMIT, bool REC>
 __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c1_sym,
                                             const StrokeParams& P, JoinSum& sum, VerbOut* o,
                                             uint32_t* last_join) {
@@ -786,7 +800,7 @@ __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c
                 if (curflat && dot(pe, ne) > 0.0f) {
                     if (!sym || !skip_impossible(prv, cur, pe, P.hw)) return false;
                     if (EMIT) {
-                        emit_step(*o, prv, cur, q, P.hw);
+                        emit_step<REC>(*o, prv, cur, q, P.hw);
                     } else {
                         sum.add(2, 0, 0, 0);
                         *last_join = PACKED_STEP;
@@ -797,7 +811,7 @@ __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c
                     uint32_t packed;
                     if (!pack_join(sj, &packed)) return false;
                     if (EMIT) {
-                        emit_general(*o, prv, cur, curflat, q, P, packed);
+                        emit_general<REC>(*o, prv, cur, curflat, q, P, packed);
                     } else {
                         sum.add(sj.vcount, sj.jtris, sj.to_f, sj.from_f);
                         *last_join = packed;
@@ -805,6 +819,7 @@ __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c
                     sym = general_sym;
                 }
             }
+            if (EMIT && REC) o->adv = o->adv + vlength(q - cur);
             prv = cur;
             cur = q;
             curflat = flat;
@@ -860,7 +875,7 @@ __global__ void __launch_bounds__(128) extra_count_kernel(StrokeArgs A, StrokeVe
             // but a clipped miter.
             const bool sym = P.line_join != LYON_JOIN_MITER_CLIP ||
                              (S.kind[v - 1] & KIND_MASK) == LYON_VERB_BEGIN;
-            ok = walk_irregular<false>(a, b, c1, sym, P, sum, nullptr, &packed);
+            ok = walk_irregular<false, false>(a, b, c1, sym, P, sum, nullptr, &packed);
         } else {
             sum.run(a.m - 1);
             const V2 before = point_before_end(a, c1), after = first_point(b);
@@ -933,9 +948,11 @@ __global__ void __launch_bounds__(256) joins_count_kernel(StrokeArgs A, StrokeVe
 }
 
 // The position of a verb's output and the edge into its first join.
+template <bool REC>
 __device__ __forceinline__ void verb_out(const StrokeArgs& A, const StrokeVerbs& S, uint32_t v,
                                          uint32_t path, VerbOut& o) {
-    o.po = path_out<true, false>(A, path);
+    o.po = path_out<true, REC>(A, path);
+    o.adv = REC ? S.adv[v - 1].w : 0.0f;
     o.vo = S.vpre[v] - S.path_v[path];
     o.io = S.ipre[v] - S.path_i[path];
     o.st = LYON_OK;
@@ -965,6 +982,7 @@ __device__ __forceinline__ void pass_run(VerbOut& o, uint32_t joins) {
 }
 
 // Output of the verbs in `extra` but for their runs.
+template <bool REC>
 __global__ void __launch_bounds__(128) extra_emit_kernel(StrokeArgs A, StrokeVerbs S) {
     if (batch_verbs(A) > S.cap) return;
     // The verbs of two runs, then, from a warp's boundary, the irregular ones.
@@ -977,7 +995,7 @@ __global__ void __launch_bounds__(128) extra_emit_kernel(StrokeArgs A, StrokeVer
         if (S.path_walk[path] || A.status[path] != LYON_OK) continue;
         const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
         VerbOut o;
-        verb_out(A, S, v, path, o);
+        verb_out<REC>(A, S, v, path, o);
         Unit a, b;
         verb_units(S.kind[v] & KIND_MASK, S.rec[v], A.points, P.tolerance, flags,
                    flags & VF_TWO ? S.cut[v] : 0u, a, b);
@@ -986,14 +1004,16 @@ __global__ void __launch_bounds__(128) extra_emit_kernel(StrokeArgs A, StrokeVer
             JoinSum none;
             none.init();
             uint32_t last;
-            if (!walk_irregular<true>(a, b, c1, true, P, none, &o, &last)) o.st = LYON_ERR_INTERNAL;
+            if (!walk_irregular<true, REC>(a, b, c1, true, P, none, &o, &last))
+                o.st = LYON_ERR_INTERNAL;
         } else {
             pass_run(o, a.m - 1);
+            if (REC) o.adv = S.adv[v].x;
             const V2 before = point_before_end(a, c1), after = first_point(b);
             if ((flags & VF_CUT) && dot(a.to - before, after - a.to) > 0.0f) {
-                emit_step(o, before, a.to, after, P.hw);
+                emit_step<REC>(o, before, a.to, after, P.hw);
             } else {
-                emit_general(o, before, a.to, (flags & VF_CUT) != 0, after, P, S.split[v]);
+                emit_general<REC>(o, before, a.to, (flags & VF_CUT) != 0, after, P, S.split[v]);
             }
         }
         if (o.st != LYON_OK) A.status[path] = o.st;
@@ -1001,6 +1021,7 @@ __global__ void __launch_bounds__(128) extra_emit_kernel(StrokeArgs A, StrokeVer
 }
 
 // Output of the join at each verb's end, one verb per thread. It is the last thing of the verb.
+template <bool REC>
 __global__ void __launch_bounds__(256) joins_emit_kernel(StrokeArgs A, StrokeVerbs S) {
     const uint32_t nv = batch_verbs(A);
     if (nv > S.cap) return;
@@ -1012,8 +1033,9 @@ __global__ void __launch_bounds__(256) joins_emit_kernel(StrokeArgs A, StrokeVer
         const uint32_t flags = S.flags[v], join = S.join[v];
         const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
         VerbOut o;
-        o.po = path_out<true, false>(A, path);
+        o.po = path_out<true, REC>(A, path);
         o.st = LYON_OK;
+        o.adv = REC ? S.adv[v].w : 0.0f;
         o.edge = true;
         uint32_t prev = PACKED_STEP;
         if (flags_nk(flags) >= 2) {
@@ -1034,9 +1056,9 @@ __global__ void __launch_bounds__(256) joins_emit_kernel(StrokeArgs A, StrokeVer
         const float4 f = S.firsts[v + 1], l = S.lasts[v];
         const V2 nxt = V2{f.x, f.y}, last = V2{l.x, l.y}, cur = last_kept(S, A.points, v);
         if (end_steps(flags, last, cur, nxt)) {
-            emit_step(o, last, cur, nxt, P.hw);
+            emit_step<REC>(o, last, cur, nxt, P.hw);
         } else {
-            emit_general(o, last, cur, (flags & VF_ENDFLAT) != 0, nxt, P, join);
+            emit_general<REC>(o, last, cur, (flags & VF_ENDFLAT) != 0, nxt, P, join);
         }
         if (o.st != LYON_OK || o.vo != end_v || o.io != end_i)
             A.status[path] = o.st != LYON_OK ? o.st : LYON_ERR_INTERNAL;
@@ -1046,6 +1068,7 @@ __global__ void __launch_bounds__(256) joins_emit_kernel(StrokeArgs A, StrokeVer
 // ---- 5. tails ----------------------------------------------------------------------------------
 
 // The TailJob of the sub-path that ends in slot v, from the recorded points.
+template <bool REC>
 __device__ __forceinline__ TailJob tail_job(const StrokeArgs& A, const StrokeVerbs& S, uint32_t v,
                                             uint32_t path, const StrokeParams& P, bool emit) {
     const uint32_t kind = S.kind[v];
@@ -1054,7 +1077,7 @@ __device__ __forceinline__ TailJob tail_job(const StrokeArgs& A, const StrokeVer
     j.path = path;
     j.flags = ((kind & KIND_MASK) == LYON_VERB_CLOSE ? TJ_CLOSED : 0u) |
               (kind & KIND_MNEC ? TJ_MNEC : 0u);
-    j.adv0 = j.adv1 = j.adv2 = 0.0f;
+    j.adv0 = j.adv1 = j.adv2 = REC ? S.adv[b].w : 0.0f;
     j.vcur = emit ? S.vpre[v] - S.path_v[path] : 0u;
     j.icur = emit ? S.ipre[v] - S.path_i[path] : 0u;
     j.base1 = j.jbase = 0;
@@ -1066,6 +1089,11 @@ __device__ __forceinline__ TailJob tail_job(const StrokeArgs& A, const StrokeVer
     const uint32_t f1 = S.flags[b + 1], fl = S.flags[v - 1];
     j.n += flags_nk(f1) + (segs > 1 ? flags_nk(S.flags[b + 2]) : 0u) + (segs > 2 ? 1u : 0u);
     j.c1 = last_kept(S, A.points, v - 1);
+    if (REC) {
+        const float4 a = S.adv[v - 1];
+        j.adv1 = a.w;
+        j.adv2 = flags_nk(fl) >= 2 ? a.z : S.adv[v - 2].w;
+    }
     if (fl & VF_ENDFLAT) j.flags |= TJ_F1;
     const float4 fs = S.firsts[b + 1], ls = S.lasts[v - 1];
     j.p1 = V2{fs.x, fs.y};
@@ -1110,7 +1138,7 @@ __device__ __forceinline__ TailJob tail_job(const StrokeArgs& A, const StrokeVer
 // Threads take the sub-path ends of a tile of TAIL_TILE slots, packed so that the warps that run
 // the caps are full: ends are a twentieth of the verbs of a drawing.
 constexpr uint32_t TAIL_TILE = 1024;
-template <bool EMIT>
+template <bool EMIT, bool REC>
 __global__ void __launch_bounds__(128) tails_kernel(StrokeArgs A, StrokeVerbs S) {
     __shared__ uint32_t ends[TAIL_TILE];
     __shared__ uint32_t count;
@@ -1129,11 +1157,11 @@ __global__ void __launch_bounds__(128) tails_kernel(StrokeArgs A, StrokeVerbs S)
             const uint32_t v = ends[i], path = S.path[v];
             if (S.path_walk[path] || (EMIT && A.status[path] != LYON_OK)) continue;
             const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
-            const TailJob j = tail_job(A, S, v, path, P, EMIT);
+            const TailJob j = tail_job<REC>(A, S, v, path, P, EMIT);
             uint32_t tv, ti;
             int st;
-            const PathOut po = path_out<EMIT, false>(A, path);
-            tail_at<false>(j, P, po, &tv, &ti, &st);
+            const PathOut po = path_out<EMIT, REC>(A, path);
+            tail_at<REC>(j, P, po, &tv, &ti, &st);
             if (EMIT) {
                 if (st != LYON_OK || j.vcur + tv != S.vpre[v + 1] - S.path_v[path] ||
                     j.icur + ti != S.ipre[v + 1] - S.path_i[path])
@@ -1345,7 +1373,7 @@ struct RunSlot {
     float hw;
     uint32_t id;         // id of its first vertex
     uint32_t pfn, pfp, edge_words;  // the edge into its first join: ids, index words
-    uint32_t pad;
+    float adv;           // the advancement before it (records)
 };
 struct RunSmem {
     RunSlot unit[WIN_UNITS];
@@ -1436,7 +1464,9 @@ __device__ __forceinline__ void write_run_indices(uint16_t* dst, uint32_t words,
 // Lane = point: tangent of the edge into the point, normal and two vertices of the join at the point
 // before, 16 bytes a lane; the indices of a run are a formula of their position and leave as
 // 16-byte stores too. Bound by instruction issue (the divisions and square roots of the normals:
-// IEEE, as lyon's) and the stores.
+// IEEE, as lyon's) and the stores. Records take a sum over the points besides, one addition after
+// another as lyon's advancement does: 32 for 32 points.
+template <bool REC>
 __global__ void __launch_bounds__(WIN_WARPS * 32) runs_kernel(StrokeArgs A, StrokeVerbs S) {
     extern __shared__ __align__(16) unsigned char run_smem[];
     const int lane = threadIdx.x & 31;
@@ -1467,8 +1497,9 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) runs_kernel(StrokeArgs A, Stro
                            flags & VF_TWO ? S.cut[v] : 0u, a, b);
                 hw = P.hw;
                 c1 = last_kept(S, A.points, v - 1);
-                verb_out(A, S, v, path, oa);
+                verb_out<REC>(A, S, v, path, oa);
                 ob = oa;
+                if (REC && b.m > 0) ob.adv = S.adv[v].x;
                 pass_run(ob, a.m - 1u);
                 const uint32_t va = ob.vo, ia = ob.io;
                 uint32_t vb = 0, ib = 0;
@@ -1513,7 +1544,8 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) runs_kernel(StrokeArgs A, Stro
         auto lay_out = [&](RunSlot& r, const Unit& x, V2 from, const VerbOut& o, uint32_t first) {
             lay_out_unit(r.u, x, from, first);
             r.hw = hw;
-            r.vout = o.po.vout + o.vo;
+            r.vout = REC ? reinterpret_cast<float2*>(o.po.rout + o.vo) : o.po.vout + o.vo;
+            r.adv = o.adv;
             r.iout = o.po.bits == 16 ? (void*)((uint16_t*)o.po.iout + o.io)
                                      : (void*)((uint32_t*)o.po.iout + o.io);
             r.id = o.po.id_base + o.vo;
@@ -1526,6 +1558,7 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) runs_kernel(StrokeArgs A, Stro
         __syncwarp();
         // ---- vertices ----
         V2 q = V2{0.0f, 0.0f}, nt = V2{0.0f, 0.0f};
+        float sum = 0.0f;  // the advancement at the last point (records)
         for (uint32_t r0 = 0; r0 < total; r0 += WIN_ROUND) {
             const uint32_t rn = min(WIN_ROUND, total - r0);
             fill_points(sm.pt, &sm.unit[0].u, sizeof(RunSlot), nunits, r0, rn, lane);
@@ -1542,7 +1575,18 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) runs_kernel(StrokeArgs A, Stro
                     qp = V2{e.x, e.y};
                 }
                 const V2 ne = q - qp;
-                nt = ne / vlength(ne);
+                const float len = vlength(ne);
+                nt = ne / len;
+                float adv = 0.0f;  // at the point before, where the join is
+                if constexpr (REC) {
+                    const uint32_t starts = __ballot_sync(FULL, k == 1u);
+#pragma unroll
+                    for (uint32_t j = 0; j < 32; ++j) {
+                        if ((starts >> j) & 1u) sum = __shfl_sync(FULL, r.adv, (int)j);
+                        if ((uint32_t)lane == j) adv = sum;
+                        sum = sum + __shfl_sync(FULL, len, (int)j);
+                    }
+                }
                 const V2 pt = V2{from_left(nt.x, old_t.x, lane), from_left(nt.y, old_t.y, lane)};
                 const float rhw = r.hw;
                 const V2 nrm = compute_normal(pt, nt);
@@ -1550,7 +1594,24 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) runs_kernel(StrokeArgs A, Stro
                 // The vertices (pn, nn) of the join at point k - 1 start at 2 (k - 2). When that is
                 // no 16-byte boundary, a lane writes its left neighbour's nn with its own pn.
                 const V2 ln = V2{__shfl_up_sync(FULL, nn.x, 1), __shfl_up_sync(FULL, nn.y, 1)};
-                if (at < rn && k > 1u) {
+                if (REC) {
+                    if (at < rn && k > 1u) {
+                        float2* dst = r.vout + 6u * (k - 2u);
+                        if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+                            float4* d = reinterpret_cast<float4*>(dst);
+                            d[0] = make_float4(pn.x, pn.y, nrm.x, nrm.y);
+                            d[1] = make_float4(adv, __uint_as_float((uint32_t)SP), nn.x, nn.y);
+                            d[2] = make_float4(-nrm.x, -nrm.y, adv, __uint_as_float((uint32_t)SN));
+                        } else {
+                            dst[0] = make_float2(pn.x, pn.y);
+                            dst[1] = make_float2(nrm.x, nrm.y);
+                            dst[2] = make_float2(adv, __uint_as_float((uint32_t)SP));
+                            dst[3] = make_float2(nn.x, nn.y);
+                            dst[4] = make_float2(-nrm.x, -nrm.y);
+                            dst[5] = make_float2(adv, __uint_as_float((uint32_t)SN));
+                        }
+                    }
+                } else if (at < rn && k > 1u) {
                     float2* dst = r.vout + 2u * (k - 2u);
                     if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
                         *reinterpret_cast<float4*>(dst) = make_float4(pn.x, pn.y, nn.x, nn.y);
@@ -1622,7 +1683,7 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
     } else {
         // Tails read the points beside the sub-paths' ends and nothing of the joins.
         const cudaStream_t t = side.fork(0, s);
-        tails_kernel<false><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
+        tails_kernel<false, false><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
         extra_count_kernel<<<grid_for(verbs_hint / 8, 128, num_sms, 8), 128, 0, s>>>(a, v);
         joins_count_kernel<<<by_verb, 256, 0, s>>>(a, v);
         side.join(0, s);
@@ -1645,27 +1706,37 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
     return cudaGetLastError();
 }
 
-cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
-                                     uint32_t verbs_hint, bool runs, int num_sms,
-                                     const SideStreams& side, cudaStream_t s) {
-    if (a.widths || a.sources || a.vertex_attrs)
-        return launch_stroke_steps_emit(a, v, verbs_hint, num_sms, side, s);
+template <bool REC>
+static void launch_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint, bool runs,
+                              int num_sms, const SideStreams& side, cudaStream_t s) {
     // The three write different parts of the output; joins and tails are short of warps and of
     // threads that agree, and fill the gaps of the runs.
     const cudaStream_t j = side.fork(0, s), t = side.fork(1, s);
     if (runs) {
-        runs_kernel<<<grid_for(verbs_hint, WIN_WARPS, num_sms, 8), WIN_WARPS * 32, RUN_SMEM, s>>>(
-            a, v);
+        runs_kernel<REC><<<grid_for(verbs_hint, WIN_WARPS, num_sms, 8), WIN_WARPS * 32, RUN_SMEM,
+                           s>>>(a, v);
         note_launches(1);
     }
     // (joins and tails are the shorter ones of a small batch, and share a stream: 1,000 paths of 16
-    // segments take 12 and 47 us there, the runs 59, the verbs apart 77)
-    extra_emit_kernel<<<grid_for(verbs_hint / 8, 128, num_sms, 8), 128, 0, j>>>(a, v);
-    joins_emit_kernel<<<grid_for(verbs_hint, 256, num_sms, 8), 256, 0, t>>>(a, v);
-    tails_kernel<true><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
+    // segments take 12 and 42 us there, the runs 58, the verbs apart 79)
+    extra_emit_kernel<REC><<<grid_for(verbs_hint / 8, 128, num_sms, 8), 128, 0, j>>>(a, v);
+    joins_emit_kernel<REC><<<grid_for(verbs_hint, 256, num_sms, 8), 256, 0, t>>>(a, v);
+    tails_kernel<true, REC><<<grid_for(verbs_hint, TAIL_TILE, num_sms, 16), 128, 0, t>>>(a, v);
     note_launches(3);
     side.join(0, s);
     side.join(1, s);
+}
+
+cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
+                                     uint32_t verbs_hint, bool runs, int num_sms,
+                                     const SideStreams& side, cudaStream_t s) {
+    if (a.widths || a.sources) return launch_stroke_steps_emit(a, v, verbs_hint, num_sms, side, s);
+    if (a.vertex_attrs) {
+        launch_stroke_advance(a, v, num_sms, side, s);
+        launch_verbs_emit<true>(a, v, verbs_hint, runs, num_sms, side, s);
+    } else {
+        launch_verbs_emit<false>(a, v, verbs_hint, runs, num_sms, side, s);
+    }
     return cudaGetLastError();
 }
 

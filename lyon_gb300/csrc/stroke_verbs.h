@@ -14,6 +14,8 @@ namespace lg {
 struct StrokeVerbs {
     uint32_t cap;          // verbs the arrays have room for (vpre and ipre: one entry more)
     float4* firsts;        // the verb's first two kept points
+    float4* adv;           // advancements (stroke_steps.cu): at the verb's last four kept points, .w
+                           // the last; for records of a verb of two runs .x at the join between
     float4* lasts;         // the kept point before the verb's last one, and the one before that
     float2* fin;           // its last kept point, where that is not its end point
     uint32_t* rec;         // first point of the verb; End/Close: the slot of the sub-path's Begin
@@ -41,7 +43,7 @@ struct StrokeVerbs {
 constexpr uint32_t STROKE_VERBS_READ = 4;    // words the host reads back
 constexpr uint32_t STROKE_VERBS_WORDS = 16;  // words in all
 // Bytes per verb of the arrays above, for their allocation.
-constexpr size_t STROKE_VERBS_BYTES = 2 * 16 + 8 + 9 * 4 + 2 + 1;
+constexpr size_t STROKE_VERBS_BYTES = 3 * 16 + 8 + 9 * 4 + 2 + 1;
 
 // Streams for kernels that run beside those of the caller's stream: fork(i, s) returns a stream
 // that continues after what is on `s`, join(i, s) makes `s` wait for it. Without streams (none
@@ -81,6 +83,8 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
 // are known, and the output of variable widths, vertex sources and attribute records.
 void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint,
                                int num_sms, const SideStreams& side, cudaStream_t s);
+void launch_stroke_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
+                           const SideStreams& side, cudaStream_t s);
 cudaError_t launch_stroke_steps_emit(const StrokeArgs& a, const StrokeVerbs& v,
                                      uint32_t verbs_hint, int num_sms, const SideStreams& side,
                                      cudaStream_t s);
