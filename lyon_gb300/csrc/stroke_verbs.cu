@@ -491,7 +491,6 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
         uint32_t path = 0, flags = 0;
         V2 c1 = V2{0.0f, 0.0f};
         float thr = 0.0f, hw = 0.0f;
-        int join = 0;
         if ((uint32_t)lane < W && v < nv) {
             const int kind = S.kind[v] & KIND_MASK;
             if (is_segment(kind)) {
@@ -508,7 +507,6 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
                     const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
                     thr = P.merge_threshold;
                     hw = P.hw;
-                    join = P.line_join;
                     flags = S.flags[v];
                     verb_units(kind, S.rec[v], A.points, P.tolerance, flags,
                                flags & VF_TURN ? S.cut[v] : 0u, a, b);
@@ -590,12 +588,13 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
                 rough |= sm.unit[slot + 1].rough;
                 bad += sm.unit[slot + 1].bad;
             }
-            // One cusp cuts the verb in two runs, unless it is split already or the sides after
-            // the join there are not symmetric (the skip test's bound wants them so).
-            if (rough || bad > 1 || (bad == 1 && (rb || join == LYON_JOIN_MITER_CLIP))) {
+            // One cusp cuts the verb in two runs, unless it is split already. (A clipped miter there
+            // leaves sides that are not symmetric, as the skip test's bound wants them:
+            // extra_count_kernel evaluates the test at the join after it.)
+            if (rough || bad > 1 || (bad == 1 && rb)) {
                 Chain c;
                 replay_chain(a, b, c1, thr, hw, c);
-                if (c.cuttable && join != LYON_JOIN_MITER_CLIP) {
+                if (c.cuttable) {
                     store_chain(S, v, path, VF_CUT | (c.at + c.gap + 1u == a.m ? VF_SECOND1 : 0u),
                                 c);
                     S.cut[v] = c.at | (c.gap << 16);
@@ -773,16 +772,16 @@ __device__ __forceinline__ void emit_step(VerbOut& o, V2 prv, V2 cur, V2 nxt, fl
 
 // The walk of one irregular verb by one thread: lyon's step over its flattened points from the
 // kept point `c1` before it (the join at c1 belongs to the verb before, the one at the last kept
-// point is not done here). Counts into `sum`, or emits through `o`. Returns false when the path
-// has to be walked as a whole: a join fails, or the skip test is not ruled out by its bound.
+// point is not done here). Counts into `sum`, or emits through `o`. Returns false, counting, when the
+// path has to be walked as a whole: a join fails, or the skip test fires or is not ruled out by its
+// bound. (After a clipped miter, whose sides are not symmetric, the test is evaluated; at the first
+// join by the verb before, first_step_skips.)
 template <bool EMIT, bool REC>
-__device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c1_sym,
-                                            const StrokeParams& P, JoinSum& sum, VerbOut* o,
-                                            uint32_t* last_join) {
-    V2 cur = c1, prv = c1;
-    bool curflat = false, sym = c1_sym;
+__device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, const StrokeParams& P,
+                                            JoinSum& sum, VerbOut* o, uint32_t* last_join) {
+    V2 cur = c1, prv = c1, jpn = c1, jnn = c1;
+    bool curflat = false, sym = true;  // of the join at prv, with the sides (jpn, jnn) if not
     uint32_t kept = 0;
-    const bool general_sym = P.line_join != LYON_JOIN_MITER_CLIP;
     const uint32_t units = b.m > 0 ? 2u : 1u;
     for (uint32_t u = 0; u < units; ++u) {
         float t = a.t0;
@@ -798,7 +797,9 @@ __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c
             if (kept > 0) {
                 const V2 pe = cur - prv, ne = q - cur;
                 if (curflat && dot(pe, ne) > 0.0f) {
-                    if (!sym || !skip_impossible(prv, cur, pe, P.hw)) return false;
+                    if (!EMIT && (sym ? !skip_impossible(prv, cur, pe, P.hw)
+                                      : skip_fires(prv, jpn, jnn, cur, q, P.hw)))
+                        return false;
                     if (EMIT) {
                         emit_step<REC>(*o, prv, cur, q, P.hw);
                     } else {
@@ -810,13 +811,15 @@ __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c
                     const SlowJoin sj = slow_join_summary(prv, cur, curflat, q, P);
                     uint32_t packed;
                     if (!pack_join(sj, &packed)) return false;
+                    jpn = sj.pn;
+                    jnn = sj.nn;
                     if (EMIT) {
                         emit_general<REC>(*o, prv, cur, curflat, q, P, packed);
                     } else {
                         sum.add(sj.vcount, sj.jtris, sj.to_f, sj.from_f);
                         *last_join = packed;
                     }
-                    sym = general_sym;
+                    sym = sj.sym;
                 }
             }
             if (EMIT && REC) o->adv = o->adv + vlength(q - cur);
@@ -835,7 +838,7 @@ __device__ __noinline__ bool walk_irregular(Unit a, const Unit& b, V2 c1, bool c
 __device__ __forceinline__ bool first_step_skips(const StrokeVerbs& S, uint32_t next, V2 cur,
                                                  const SlowJoin& sj, float hw) {
     const uint32_t f = S.flags[next];
-    if (sj.sym || (f & VF_IRR) || !(f & VF_FLAT1) || flags_nk(f) < 2) return false;
+    if (sj.sym || !(f & VF_FLAT1) || flags_nk(f) < 2) return false;
     const float4 q = S.firsts[next];
     const V2 q1 = V2{q.x, q.y}, q2 = V2{q.z, q.w};
     if (!(dot(q1 - cur, q2 - q1) > 0.0f)) return false;
@@ -871,11 +874,7 @@ __global__ void __launch_bounds__(128) extra_count_kernel(StrokeArgs A, StrokeVe
         const V2 c1 = last_kept(S, A.points, v - 1);
         uint32_t packed = PACKED_STEP;
         if (flags & VF_IRR) {
-            // The join at a Begin point has symmetric sides; so has every other general join
-            // but a clipped miter.
-            const bool sym = P.line_join != LYON_JOIN_MITER_CLIP ||
-                             (S.kind[v - 1] & KIND_MASK) == LYON_VERB_BEGIN;
-            ok = walk_irregular<false, false>(a, b, c1, sym, P, sum, nullptr, &packed);
+            ok = walk_irregular<false, false>(a, b, c1, P, sum, nullptr, &packed);
         } else {
             sum.run(a.m - 1);
             const V2 before = point_before_end(a, c1), after = first_point(b);
@@ -1004,7 +1003,7 @@ __global__ void __launch_bounds__(128) extra_emit_kernel(StrokeArgs A, StrokeVer
             JoinSum none;
             none.init();
             uint32_t last;
-            if (!walk_irregular<true, REC>(a, b, c1, true, P, none, &o, &last))
+            if (!walk_irregular<true, REC>(a, b, c1, P, none, &o, &last))
                 o.st = LYON_ERR_INTERNAL;
         } else {
             pass_run(o, a.m - 1);

@@ -328,3 +328,15 @@ def test_counts_finished_by_one_block(ctx, n):
     opts = options(rng, batch.num_paths)
     check(ctx, batch, opts)
     check(ctx, batch, opts, 16, T.INDEX_PER_PATH, 65500)
+
+
+@pytest.mark.parametrize("limit", [1.0, 1.05, 1.5, 4.0])
+@pytest.mark.parametrize("width", [0.3, 5.0, 40.0])
+def test_clipped_miters(ctx, limit, width):
+    # Clipped miters leave sides that are not symmetric, before runs, at cusps and inside irregular
+    # verbs: the skip test of the step after each is evaluated, not ruled out by its bound.
+    batch = rough_paths(600, int(limit * 100 + width))
+    opts = options(np.random.default_rng(5), batch.num_paths, join=1)
+    opts["miter_limit"] = limit
+    opts["line_width"] = width
+    check(ctx, batch, opts)
