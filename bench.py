@@ -186,15 +186,8 @@ def profiled_figure(name, key):
 
 
 def profiled_traffic_per_vertex():
-    """DRAM bytes per output vertex of the emit kernel from the committed ncu summary, if any."""
-    p = os.path.join(ROOT, "profiles", "stroke_emit_batched_stroke.md")
-    try:
-        for line in open(p):
-            if line.startswith("dram_bytes_per_output_vertex:"):
-                return float(line.split(":", 1)[1].strip())
-    except OSError:
-        pass
-    return None
+    """DRAM bytes per output vertex of the emit kernels from the committed ncu summary, if any."""
+    return profiled_figure("stroke_emit_by_verb.md", "dram_bytes_per_output_vertex")
 
 
 def _oracle_rate(kind, batch, opts, n, threads, ties=None):
@@ -399,7 +392,7 @@ def main():
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": (tpv * verts_per_step) if tpv is not None else None,
-                "kernel": "stroke_kernel<true> (emit)",
+                "kernel": "runs_kernel and, beside it, joins, cusps and tails (emit)",
                 "algorithmic_bytes": in_bytes + out_bytes,
                 "emit_ms": emit_s * 1e3}
 
@@ -475,9 +468,8 @@ def run_fill(ctx, args, T, world, batch=None):
         opts = np.zeros(1, dtype=FILL_OPTIONS_DTYPE)
         opts[0] = (0.1, rule, 0, 1)
         od = T.upload_options(opts, 0)
-        # The fill autotuner picks blocks per SM and sweepers per warp on a sample of half the
-        # batch: a sample with few paths per sweeper favours one sweeper per warp, which is 1.6x
-        # slower on the whole batch (measured with a 20,000-path sample).
+        # The fill autotuner picks blocks per SM (and the threads of a warp for tiny paths, of which
+        # this batch has none) on a sample of half the batch.
         tune = None
         if not args.profile_fill:
             best = _native.CFillTuning()
@@ -529,9 +521,9 @@ def run_fill(ctx, args, T, world, batch=None):
         # output vertices and indices, per-path descriptors) over the sweep's event time.
         alg = (batch.input_bytes(options_bytes_per_path=0) + 16 + v * 8 +
                res.total_indices * 4 + 16 * batch.num_paths)
-        tpp = profiled_figure("fill_sweep_glyph_fill.md", "dram_bytes_per_path")
+        tpp = profiled_figure("fill_warp_glyph_fill.md", "dram_bytes_per_path")
         entry["roofline"] = roofline_entry(
-            alg, statistics.median(sweep_ms) / 1e3, "fill_sweep_kernel",
+            alg, statistics.median(sweep_ms) / 1e3, "fill_warp_kernel",
             tpp * batch.num_paths if tpp is not None else None)
         n = min(20_000, batch.num_paths)
         rate, cv, dt = _oracle_rate("fill", batch, opts, n, threads)
@@ -589,7 +581,7 @@ def run_variable_width(ctx, args, T):
     # whole call (both passes of the sequential stepper, the scan).
     alg = (batch.input_bytes(options_bytes_per_path=24) + 4 * len(batch.points) +
            res.total_vertices * 8 + res.total_indices * 4 + 16 * batch.num_paths)
-    out["roofline"] = roofline_entry(alg, ms / 1e3, "whole call (stroke_seq_kernel count and emit)")
+    out["roofline"] = roofline_entry(alg, ms / 1e3, "whole call (steps_kernel count and emit)")
     threads = os.cpu_count() or 1
     n = min(20_000, batch.num_paths)
     sub = batch.head(n)
@@ -647,7 +639,7 @@ def run_custom_attributes(ctx, args, T, baseline=True):
     alg = (batch.input_bytes(options_bytes_per_path=24) + 8 * len(batch.points) +
            res.total_vertices * (8 + 12 + 8) + res.total_indices * 4 + 16 * batch.num_paths)
     out["roofline"] = roofline_entry(alg, ms / 1e3,
-                                     "whole call (warp count, sequential emit, interpolation)")
+                                     "whole call (count, steps_kernel emit, interpolation)")
     if not baseline:
         return out
     threads = os.cpu_count() or 1
@@ -861,9 +853,9 @@ def run_polylines(ctx, args, T):
                  "gpu_launches": ctx.lib.lyon_gpu_kernel_launches() - launches0}
         alg = (batch.input_bytes(options_bytes_per_path=24) + res.total_vertices * 8 +
                res.total_indices * 4 + 16 * batch.num_paths)
-        tpv = profiled_figure("stroke_emit_map_polylines_300k.md", "dram_bytes_per_output_vertex")
+        tpv = profiled_figure("stroke_emit_by_verb.md", "map_dram_bytes_per_output_vertex")
         entry["roofline"] = roofline_entry(
-            alg, statistics.median(emit_ms) / 1e3, "stroke_kernel<true> (emit: warp walk and one-thread short paths)",
+            alg, statistics.median(emit_ms) / 1e3, "joins_emit_kernel and, beside it, tails_kernel (emit)",
             tpv * res.total_vertices if tpv is not None else None)
         if tol == 0.1:
             n = batch.num_paths  # the whole batch: well under a second on the host cores

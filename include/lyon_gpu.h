@@ -243,7 +243,7 @@ int lyon_gpu_stroke_paths_attributes(lyon_gpu_context* ctx, const lyon_path_batc
  * interpolated along curves). `widths` (device memory) holds one factor per point of the batch,
  * indexed like `points`; entries of control points and of Close's repeated point are not read.
  * `vertex_attributes` non-zero writes lyon_stroke_vertex records instead of positions. The rest
- * is as for lyon_gpu_stroke_paths. Each path is stroked by one thread. */
+ * is as for lyon_gpu_stroke_paths. */
 int lyon_gpu_stroke_paths_variable_width(lyon_gpu_context* ctx, const lyon_path_batch* batch,
                                          const float* widths,
                                          const lyon_stroke_options* options,
@@ -686,7 +686,8 @@ int lyon_gpu_coverage_compare(const float* boxes, uint32_t num_paths, uint32_t g
 
 /* ---- Stroke launch settings and autotuner (no lyon counterpart) ---------------------------- */
 
-/* Runtime settings of the stroke kernels on a context. */
+/* Runtime settings of the stroke kernels that take a path as a whole, which are for the paths that the
+ * verb-parallel stroke leaves. */
 typedef struct lyon_gpu_stroke_tuning {
     uint32_t long_path_points;  /* paths with more points are scheduled first (so that no long
                                    path is left running alone at the end of a launch);
@@ -713,13 +714,13 @@ int lyon_gpu_autotune_stroke(lyon_gpu_context* ctx, const lyon_path_batch* batch
                              uint32_t sample_paths, lyon_gpu_stroke_tuning* best,
                              float* times_ms, uint32_t* num_candidates);
 
-/* Runtime settings of the fill sweep on a context: lyon's sweep of one path runs on one thread
- * (a sweeper); a one-warp block holds up to 32 of them. */
+/* Runtime settings of the fill sweep on a context: lyon's sweep of one path runs on one warp (a
+ * block). In batches of 16,384 or more paths of lines with fewer than 8 points those paths are swept
+ * by one thread each, several of a block. */
 typedef struct lyon_gpu_fill_tuning {
     uint32_t blocks_per_sm; /* sweep blocks per SM; 0: the default (16) */
-    uint32_t lanes;         /* sweepers per block: 1 (a path owns its warp) to 32 (a warp shared by
-                               32 paths, which share its instruction fetch and issue slots);
-                               0: chosen per launch (1 below two paths per block, else up to 12) */
+    uint32_t lanes;         /* threads of a block that sweep tiny paths: 1 to 32; 0: chosen per launch
+                               from its paths per block, up to 12 */
 } lyon_gpu_fill_tuning;
 
 int lyon_gpu_set_fill_tuning(lyon_gpu_context* ctx, const lyon_gpu_fill_tuning* tuning);
@@ -728,11 +729,9 @@ int lyon_gpu_get_fill_tuning(lyon_gpu_context* ctx, lyon_gpu_fill_tuning* tuning
 /* Times the batched fill (device buffers, u32 per-path indices) on the first `sample_paths`
  * paths of `batch` (0: all) for each candidate setting — blocks_per_sm in {16, 8} x lanes in
  * {1, 4, 8, 12, 16} — and keeps the fastest on the context, so that later calls on paths of the
- * same size distribution use it: the split between a path owning its warp and paths sharing one.
- * `best` receives the choice, `times_ms` (optional, 10 entries, lanes varying fastest) the
- * candidates' times, `num_candidates` the count. Outputs do not depend on the settings. The
- * sample must give each sweeper about as many paths as the whole batch will: with too few
- * paths per sweeper, a path owning its warp wins on the sample and loses on the batch. */
+ * same size distribution use it. `best` receives the choice, `times_ms` (optional, 10 entries, lanes
+ * varying fastest) the candidates' times, `num_candidates` the count. Outputs do not depend on the
+ * settings. */
 int lyon_gpu_autotune_fill(lyon_gpu_context* ctx, const lyon_path_batch* batch,
                            const lyon_fill_options* options, uint32_t num_options,
                            uint32_t sample_paths, lyon_gpu_fill_tuning* best, float* times_ms,
