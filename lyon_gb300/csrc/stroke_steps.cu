@@ -121,6 +121,26 @@ __device__ __forceinline__ uint32_t verb_edges(const StrokeArgs& A, const Stroke
     return M;
 }
 
+// Running f32 sums over four-point words of shared memory, one addition after another: sums[i] =
+// sums[i - 1] + lengths[i], from `adv`. Every lane runs it, lane 0 writes. A word is loaded while the
+// one before it is added.
+__device__ __forceinline__ float running_sums(const float4* lengths, float4* sums, uint32_t words,
+                                              float adv, int lane) {
+    float4 next = words > 0 ? lengths[0] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (uint32_t w = 0; w < words; ++w) {
+        float4 x = next;
+        if (w + 1u < words) next = lengths[w + 1u];
+        x.x = adv + x.x;
+        x.y = x.x + x.y;
+        x.z = x.y + x.z;
+        x.w = x.z + x.w;
+        adv = x.w;
+        if (lane == 0) sums[w] = x;
+    }
+    return adv;
+}
+
 // Paths of more verbs than this are taken by blocks (below), the others by warps.
 constexpr uint32_t ADVANCE_LONG = 64;
 
@@ -132,9 +152,13 @@ __device__ __forceinline__ void keep_advancement(float* out, uint32_t e, uint32_
     if (first && e + 1u == first) out[0] = adv;
 }
 
-// Warp per path. Bound by the sum's chain, 32 additions for 32 points.
+// Warp per path. Bound by the sum's chain, 32 additions for 32 points, which run on words of shared
+// memory (a shuffle per addition took 0.76 ms for 20,000 paths, this 0.62).
 __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs S) {
+    __shared__ float4 lengths[4][8], sums[4][8];
     const int lane = threadIdx.x & 31;
+    float4* const len4 = lengths[threadIdx.x >> 5];
+    float4* const sum4 = sums[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     if (batch_verbs(A) > S.cap || S.words[1] != 0) return;
@@ -158,25 +182,25 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
                 }
                 st.kept += verb_edges(A, S, v, k, P, lane, [&](uint32_t e, uint32_t cnt, float len,
                                                                uint32_t M, uint32_t m1) {
-                    float mine = 0.0f;
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; ++j) {
-                        const float x = __shfl_sync(FULL, len, (int)j);
-                        st.adv = st.adv + (j < cnt ? x : 0.0f);
-                        if ((uint32_t)lane == j) mine = st.adv;
-                    }
-                    keep_advancement(out + 4 * (size_t)v, e, M, runs ? m1 : 0u, mine);
+                    reinterpret_cast<float*>(len4)[lane] = (uint32_t)lane < cnt ? len : 0.0f;
+                    __syncwarp();
+                    st.adv = running_sums(len4, sum4, (cnt + 3u) / 4u, st.adv, lane);
+                    __syncwarp();
+                    keep_advancement(out + 4 * (size_t)v, e, M, runs ? m1 : 0u,
+                                     reinterpret_cast<const float*>(sum4)[lane]);
+                    __syncwarp();
                 });
             }
         }
     }
 }
 
-// Block per long path: the lengths of a window of verbs by all its warps, then the sum over them by
-// one (one warp for both took 1.9 ms for a path of 35,000 points).
+// Block per long path: the lengths of a window of verbs by all its warps, then the sums over them by
+// one (one warp for both took 1.9 ms for a path of 35,000 points; with the four places of each verb
+// kept during the sum 0.93 ms, taken from the stored sums afterwards, lane = verb, 0.74).
 constexpr uint32_t ADVANCE_ROOM = 4096;
 __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeVerbs S) {
-    __shared__ float4 room[ADVANCE_ROOM / 4];
+    __shared__ float4 room[ADVANCE_ROOM / 4], sums[ADVANCE_ROOM / 4];
     __shared__ uint32_t first[33];
     __shared__ int kinds[32];
     __shared__ uint32_t split[32];  // edges of the first of two runs, else 0
@@ -232,6 +256,8 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                            [&](uint32_t e, uint32_t, float x, uint32_t M, uint32_t) {
                                if (e < M) len[first[i] + e] = x;
                            });
+                const uint32_t m = (uint32_t)kinds[i] >> 4;  // (zeros up to the word's end)
+                if (m + (uint32_t)lane < ((m + 3u) & ~3u)) len[first[i] + m + lane] = 0.0f;
             }
             __syncthreads();
             if (warp == 0 && n == 0) {
@@ -247,38 +273,40 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                     keep_advancement(out + 4 * (size_t)base, e, M, runs ? m1 : 0u, mine);
                 });
             }
-            for (uint32_t i = 0; warp == 0 && i < n; ++i) {
-                const uint32_t v = base + i, m = (uint32_t)kinds[i] >> 4;
-                const int k = kinds[i] & 15;
-                if (!is_segment(k)) {
-                    advance_special(A, S, v, k & 7, P, st, lane);
+            // The sums of the window's rows of run verbs; lane = verb then takes its four.
+            const int mine = warp == 0 && (uint32_t)lane < n ? kinds[lane] : KIND_NONE;
+            const uint32_t special = __ballot_sync(FULL, !is_segment(mine & 15));
+            for (uint32_t i = 0; warp == 0 && i < n;) {
+                if ((special >> i) & 1u) {
+                    advance_special(A, S, base + i, (kinds[i] & 15) & 7, P, st, lane);
+                    ++i;
                     continue;
                 }
-                float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = st.adv;
-                const float4* w = room + first[i] / 4u;
-                uint32_t j = 0;
-                const uint32_t m1 = split[i];
-                float between = 0.0f;
-                for (; j + 4u <= m; j += 4u) {
-                    const float4 x = w[j / 4u];
-                    a0 = a3 + x.x;
-                    a1 = a0 + x.y;
-                    a2 = a1 + x.z;
-                    a3 = a2 + x.w;
-                    if (m1 > j && m1 <= j + 4u)
-                        between = m1 == j + 1u ? a0 : m1 == j + 2u ? a1 : m1 == j + 3u ? a2 : a3;
+                const uint32_t rest = special >> i;
+                const uint32_t end = rest ? min(n, i + (uint32_t)__ffs((int)rest) - 1u) : n;
+                const uint32_t w0 = first[i] / 4u;
+                const uint32_t w1 = (first[end - 1u] + ((uint32_t)kinds[end - 1u] >> 4) + 3u) / 4u;
+                const float start = st.adv;
+                st.adv = running_sums(room + w0, sums + w0, w1 - w0, start, lane);
+                __syncwarp();
+                const float* sum = reinterpret_cast<const float*>(sums);
+                uint32_t m = 0;
+                if ((uint32_t)lane >= i && (uint32_t)lane < end) {
+                    m = (uint32_t)mine >> 4;
+                    const uint32_t f = first[lane], m1 = split[lane];
+                    const float before =
+                        (uint32_t)lane == i ? start
+                                            : sum[first[lane - 1] + ((uint32_t)kinds[lane - 1] >> 4) - 1u];
+                    float a[4];
+#pragma unroll
+                    for (uint32_t c = 0; c < 4; ++c)
+                        a[c] = m + c >= 4u ? sum[f + m + c - 4u] : m + c == 3u ? before : 0.0f;
+                    if (m1) a[0] = sum[f + m1 - 1u];
+                    advancements(S)[base + lane] = make_float4(a[0], a[1], a[2], a[3]);
                 }
-                for (; j < m; ++j) {
-                    const float x = len[first[i] + j];
-                    a0 = a1;
-                    a1 = a2;
-                    a2 = a3;
-                    a3 = a3 + x;
-                    if (m1 == j + 1u) between = a3;
-                }
-                st.adv = a3;
-                st.kept += m;
-                if (lane == 0) advancements(S)[v] = make_float4(m1 ? between : a0, a1, a2, a3);
+                st.kept += __reduce_add_sync(FULL, m);
+                __syncwarp();
+                i = end;
             }
             base += n > 0 ? n : 1u;
         }
@@ -641,7 +669,7 @@ uint32_t blocks_for(uint32_t items, uint32_t per_block, int num_sms, uint32_t wa
 }  // namespace
 
 // Side by side: the long paths are few blocks, each bound by its chain of additions (20,000 paths with
-// records: 0.93 and 0.76 ms one after the other).
+// records: 0.74 and 0.62 ms one after the other).
 void launch_stroke_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
                            const SideStreams& side, cudaStream_t s) {
     const cudaStream_t l = side.fork(0, s);

@@ -30,7 +30,7 @@
 //
 // Measured, whole calls on one GB300, against the warp-per-path walk for every path: 200,000 curve
 // paths (0.47 G vertices) 36.1 -> 8.4 ms, 400,001 map polylines 15.6 -> 1.75 ms, attribute records on
-// 20,000 paths 6.4 -> 2.9 ms (by lyon's stepper, a verb per thread, 4.6), 10,000 curve paths
+// 20,000 paths 6.4 -> 2.5 ms (by lyon's stepper, a verb per thread, 4.6), 10,000 curve paths
 // from and to pinned host memory 9.5 -> 3.6 ms, 1,000 paths of 16 segments 287 -> 241 us, one such
 // path from and to host arrays 231 -> 157 us. The walk was bound by the latency of one warp's
 // chunks (6,000 to 14,000 cycles for 32 points, its code larger than the instruction cache, the
