@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
     float4* const sum4 = sums[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    if (batch_verbs(A) > S.cap || S.words[1] != 0) return;
+    if (unfit(S, batch_verbs(A))) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
     const bool runs = !A.widths && !A.sources;  // records: written run by run (stroke_verbs.cu)
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
     __shared__ uint32_t window;
     float* len = reinterpret_cast<float*>(room);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (batch_verbs(A) > S.cap || S.words[1] != 0) return;
+    if (unfit(S, batch_verbs(A))) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
     const bool runs = !A.widths && !A.sources;
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(128) steps_kernel(StrokeArgs A, StrokeVerbs S)
     __shared__ uint16_t list[STEP_TILE];
     __shared__ uint32_t count[3];
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap || S.words[1] != 0) return;
+    if (unfit(S, nv)) return;
     for (uint32_t tile = blockIdx.x * STEP_TILE; tile < nv; tile += gridDim.x * STEP_TILE) {
         for (int kind = 0; kind < 3; ++kind) {
             __syncthreads();
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(128) steps_kernel(StrokeArgs A, StrokeVerbs S)
 // Every verb's state against the one the verb before left.
 __global__ void __launch_bounds__(256) check_states_kernel(StrokeArgs A, StrokeVerbs S) {
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap || S.words[1] != 0) return;
+    if (unfit(S, nv)) return;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv;
          v += gridDim.x * blockDim.x) {
         const int kind = S.kind[v] & KIND_MASK;

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(256) turns_kernel(StrokeArgs A, StrokeVerbs S)
     __shared__ uint32_t list[TURN_TILE];
     __shared__ uint32_t count;
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap) return;
+    if (unfit(S, nv)) return;
     for (uint32_t tile = blockIdx.x * TURN_TILE; tile < nv; tile += gridDim.x * TURN_TILE) {
         __syncthreads();
         if (threadIdx.x == 0) count = 0;
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap) return;
+    if (unfit(S, nv)) return;
     const uint32_t W = window_verbs(nv, nwarps);
     for (uint32_t w0 = warp * W; w0 < nv; w0 += nwarps * W) {
         const uint32_t v = w0 + (uint32_t)lane;
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
 // A verb whose end point merged leaves the next verb another point to start from than
 // walk_kernel took: its chain again from there.
 __global__ void __launch_bounds__(128) drops_kernel(StrokeArgs A, StrokeVerbs S) {
-    if (batch_verbs(A) > S.cap) return;
+    if (unfit(S, batch_verbs(A))) return;
     const uint32_t n = S.words[4];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t v = S.drops[i], next = v + 1, path = S.path[v];
@@ -855,7 +855,7 @@ __device__ __forceinline__ bool end_steps(uint32_t flags, V2 last, V2 cur, V2 nx
 // ipre (triangles), and in `split` the join between the two runs, or an irregular verb's last
 // interior join.
 __global__ void __launch_bounds__(128) extra_count_kernel(StrokeArgs A, StrokeVerbs S) {
-    if (batch_verbs(A) > S.cap) return;
+    if (unfit(S, batch_verbs(A))) return;
     // The verbs of two runs, then, from a warp's boundary, the irregular ones.
     const uint32_t n2 = S.words[6], start = (n2 + 31u) & ~31u, n = start + S.words[7];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -910,7 +910,7 @@ __device__ __forceinline__ uint32_t last_interior(const StrokeVerbs& S, uint32_t
 // (about a thousand instructions with a round join), which every lane of a warp runs at once.
 __global__ void __launch_bounds__(256) joins_count_kernel(StrokeArgs A, StrokeVerbs S) {
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap) return;
+    if (unfit(S, nv)) return;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv;
          v += gridDim.x * blockDim.x) {
         if (!is_segment(S.kind[v] & KIND_MASK)) continue;
@@ -1142,7 +1142,7 @@ __global__ void __launch_bounds__(128) tails_kernel(StrokeArgs A, StrokeVerbs S)
     __shared__ uint32_t ends[TAIL_TILE];
     __shared__ uint32_t count;
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap) return;
+    if (unfit(S, nv)) return;
     for (uint32_t tile = blockIdx.x * TAIL_TILE; tile < nv; tile += gridDim.x * TAIL_TILE) {
         __syncthreads();
         if (threadIdx.x == 0) count = 0;
@@ -1200,7 +1200,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) verb_scan_kernel(StrokeArgs A, S
     __shared__ uint32_t tile_s;
     __shared__ unsigned long long prefix_s[2];
     const uint32_t nv = batch_verbs(A);
-    if (nv > S.cap) return;
+    // (The look-back may set words[1] while other blocks start: every thread of a block goes by one
+    // reading, and a scan that failed is not used.)
+    if (__syncthreads_or(unfit(S, nv))) return;
     const uint32_t num_tiles = (nv + SCAN_TILE - 1) / SCAN_TILE;
     for (;;) {
         __syncthreads();
@@ -1246,11 +1248,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) verb_scan_kernel(StrokeArgs A, S
 
 __global__ void __launch_bounds__(256) paths_kernel(StrokeArgs A, StrokeVerbs S) {
     const uint32_t v0 = A.verb_offsets[0], nv = batch_verbs(A);
-    const bool unfit = nv > S.cap || S.words[1] != 0;
+    const bool none = unfit(S, nv);
     for (uint32_t path = blockIdx.x * blockDim.x + threadIdx.x; path < A.num_paths;
          path += gridDim.x * blockDim.x) {
         uint32_t vc = 0, ic = 0;
-        if (!unfit) {
+        if (!none) {
             const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
             if (nv > 0) {
                 const uint32_t pv = S.vpre[s0], pi = S.ipre[s0];
@@ -1277,9 +1279,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) finish_kernel(StrokeArgs A, Stro
                                                               StrokeFinish F) {
     __shared__ uint32_t failed_s;
     const uint32_t v0 = A.verb_offsets[0], nv = batch_verbs(A);
+    const bool none = unfit(S, nv);
     if (threadIdx.x == 0) failed_s = 0;
     __syncthreads();
-    if (VERBS && nv <= S.cap) {
+    if (VERBS && !none) {
         unsigned long long pa = 0, pb = 0;
         for (uint32_t at = 0; at < nv; at += SCAN_TILE) {
             const uint32_t base = at + threadIdx.x * SCAN_ITEMS;
@@ -1312,14 +1315,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) finish_kernel(StrokeArgs A, Stro
         }
         __syncthreads();
     }
-    const bool unfit = nv > S.cap || S.words[1] != 0;
     unsigned long long pa = 0, pb = 0;
     for (uint32_t at = 0; at < A.num_paths; at += SCAN_THREADS) {
         const uint32_t path = at + threadIdx.x;
         uint32_t vc = 0, ic = 0;
         if (path < A.num_paths) {
             int32_t status = LYON_OK;
-            if (!unfit) {
+            if (!none) {
                 const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
                 if (nv > 0) {
                     const uint32_t pv = S.vpre[s0], pi = S.ipre[s0];
