@@ -11,9 +11,10 @@
 // With a fixed width the count phase of stroke_verbs.cu has the counts, and has ruled out all that
 // would make the state depend on more. With a variable width the stepper counts as well, and the
 // claim is checked: a hash of the state a thread started its verb with has to equal the one the
-// thread of the verb before ended with, over all verbs of the path, or the path is stroked by one
-// thread as a whole (stroke_seq.cu), as are the paths that stroke_verbs.cu leaves out. (A clipped
-// miter moves side points of the joins after it, so those paths usually go that way.)
+// thread of the verb before ended with, over all verbs of the path, and each sub-path's end has to
+// leave the advancement that the next one started with, or the path is stroked by one thread as a
+// whole (stroke_seq.cu), as are the paths that stroke_verbs.cu leaves out. (A clipped miter moves
+// side points of the joins after it, so those paths usually go that way.)
 //
 // The advancement kernels also serve attribute records, which stroke_verbs.cu writes run by run.
 //
@@ -56,7 +57,8 @@ __device__ __forceinline__ void advance_special(const StrokeArgs& A, const Strok
         st.kept = 1;
         if (lane == 0) out[3] = st.adv;
     } else if (is_end(kind)) {
-        // end_with_caps carries the last advancement on (stroke.rs:1359).
+        // end_with_caps carries the last advancement on (stroke.rs:1359). (With a variable width
+        // step_verb checks it.)
         if (st.kept >= 2 && !(kind == LYON_VERB_CLOSE && st.kept > 2)) st.start = st.adv;
     } else if (is_segment(kind)) {
         const uint32_t flags = S.flags[v];
@@ -606,8 +608,15 @@ __device__ __forceinline__ void step_verb(const StrokeArgs& A, const StrokeVerbs
             ni0 = s.ni;
             if (VW) state_hashes(S)[v].x = state_hash(T, s.id_base + s.nv);
         }
-        float start_adv = 0.0f;
+        float start_adv = ADV ? advancement_back(S, b, 0) : 0.0f;
         stepper_end<VW>(T, keep, kind == LYON_VERB_CLOSE, P, s, &status, &start_adv);
+        // Where the path's next sub-path starts, against what advance_special took: a skipped step
+        // replaces a point of a variable-width stroke, and the sum over its points is another one.
+        // (Only records show it.)
+        if (VW && !EMIT && A.vertex_attrs && v + 1u < A.verb_offsets[path + 1] - A.verb_offsets[0] &&
+            (S.kind[v + 1] & KIND_MASK) == LYON_VERB_BEGIN &&
+            !(start_adv == advancement_back(S, v + 1, 0)))
+            leave_to_walk(S, path);
     }
     if (EMIT) {
         if (s.overflow && status == LYON_OK) status = LYON_ERR_INTERNAL;
