@@ -2128,8 +2128,9 @@ int lyon_gpu_flatten_paths(lyon_gpu_context* ctx, const lyon_path_batch* batch, 
     a.tolerance = tolerance;
     a.counts = as<uint32_t>(ctx->flat_counts);
     a.firsts = a.counts + nv;
-    // Verbs of no path (before the first offset) have no points.
-    cudaMemsetAsync(a.firsts, 0xFF, (size_t)nv * 4, s);
+    // Verbs of no path (before the first offset) have no points: counts and firsts alike.
+    static_assert(lg::FLATTEN_NO_POINTS == 0, "cleared with the counts");
+    cudaMemsetAsync(a.counts, 0, (size_t)nv * 8, s);
     if (batch->num_paths > 0 &&
         !set_err(ctx, "flatten counts", lg::launch_flatten_counts(a, ctx->num_sms, s)))
         return LYON_ERR_CUDA;

@@ -22,7 +22,7 @@ struct FlattenArgs {
     float* out_points;         // point pass output
 };
 
-constexpr uint32_t FLATTEN_NO_POINTS = 0xFFFFFFFFu;
+constexpr uint32_t FLATTEN_NO_POINTS = 0;  // (a path's first point is its Begin's)
 
 cudaError_t launch_flatten_counts(const FlattenArgs& a, int num_sms, cudaStream_t s);
 // Points of the verbs [0, num_verbs) that the count pass gave a first point.
