@@ -50,8 +50,11 @@ __global__ void __launch_bounds__(256) flatten_count_kernel(FlattenArgs A) {
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    // (The arrays end with the last path's verbs, also where offsets run backwards.)
+    const uint32_t v_last = A.verb_offsets[A.num_paths];
     for (uint32_t path = warp; path < A.num_paths; path += nwarps) {
-        const uint32_t v_begin = A.verb_offsets[path], v_end = A.verb_offsets[path + 1];
+        const uint32_t v_begin = A.verb_offsets[path];
+        const uint32_t v_end = min(A.verb_offsets[path + 1], v_last);
         uint32_t pc = A.point_offsets[path];
         const uint32_t p_end = A.point_offsets[path + 1];
         for (uint32_t vi = v_begin; vi < v_end; vi += 32) {

@@ -53,3 +53,20 @@ def test_view_after_a_larger_batch(ctx, first, last):
     assert not offsets[:v0 + 1].any()
     assert np.array_equal(offsets[v0:], want_offsets[v0:v1 + 1] - want_offsets[v0])
     assert np.array_equal(points, want[want_offsets[v0]:want_offsets[v1]])
+
+
+def test_offsets_that_run_backwards(ctx):
+    # The batch ends before its first path does: verbs past the end have no place in the outputs.
+    batch, _ = workloads.batched_stroke(40, seed=3)
+    db = T.DeviceBatch.upload(batch, 0)
+    want, want_offsets = flatten(ctx, db, 0.05, len(batch.verbs))
+    end = int(batch.verb_offsets[5])
+    vo = np.array([0, batch.verb_offsets[30], end], np.int32)
+    po = np.array([0, batch.point_offsets[30], batch.point_offsets[5]], np.int32)
+    import torch
+    db.verb_offsets, db.point_offsets = torch.from_numpy(vo).cuda(), torch.from_numpy(po).cuda()
+    db.num_paths = 2
+    torch.cuda.synchronize()
+    points, offsets = flatten(ctx, db, 0.05, end)
+    assert np.array_equal(offsets, want_offsets[:end + 1])
+    assert np.array_equal(points, want[:want_offsets[end]])
