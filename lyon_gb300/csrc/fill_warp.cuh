@@ -361,6 +361,7 @@ __device__ __noinline__ uint32_t insert_event(SweepSmem& S, const InsertArgs& A)
 #pragma unroll 1
     for (;;) {
         if (current == NONE) {
+            __syncwarp();
             if (lane == 0) e.link[prev].y = idx;
             break;
         }
@@ -1280,8 +1281,10 @@ struct WarpFiller {
                 fail(FILL_ERR_HEAP);
                 return;
             }
+            uint2 s = make_uint2(0u, 0u);
+            if (live) s = spans[idx];
+            __syncwarp();  // two lanes may have the same span, and one of them writes it
             if (live) {
-                const uint2 s = spans[idx];
                 const uint32_t again = (ve_n > 0 && i > 0 && idx == ve_span0 ? 1u : 0u) +
                                        (ve_n > 1 && i > 1 && idx == ve_span1 ? 1u : 0u);
                 const int side = i == 0 && !end ? ve_side0 : LEFT;
