@@ -401,7 +401,9 @@ __device__ __forceinline__ void feed_begin(Stepper<VW>& T, const StrokeArgs& A,
 }
 
 // Steps the last kept points before the verb in slot `v`: at least four, or all from the
-// sub-path's Begin.
+// sub-path's Begin. Goes back over six verbs at most: each keeps a point at least, and of two in a
+// row the end point of one at least (drops_kernel), from which the steps can start when four points
+// follow it.
 template <bool VW, bool KEEP, class SK>
 __device__ __noinline__ void warm_up(Stepper<VW>& St, const StrokeArgs& A, const StrokeVerbs& S,
                                      uint32_t v, float lw, const StrokeParams& P, SK& sink,
@@ -414,12 +416,13 @@ __device__ __noinline__ void warm_up(Stepper<VW>& St, const StrokeArgs& A, const
         const uint32_t f = S.flags[u], nk = flags_nk(f);
         // Of a verb whose steps are all kept the last ones are enough, unless a cusp is near
         // (its sides hang on the points before it).
+        const bool end = have >= 4u && !(f & VF_MERGED);
         const uint32_t need = have >= 4u ? 1u : 4u - have;
-        if (!(f & VF_IRR) && (nk >= need || nk >= 3u)) {
+        if (end || (!(f & VF_IRR) && (nk >= need || nk >= 3u))) {
             VerbFeed x;
             load_feed<VW>(x, A, S, u, lw, P.tolerance);
             const uint32_t all = x.a.m + x.b.m, cut = f & VF_CUT ? S.cut[u] : 0u;
-            if (all >= need && cut <= 0xFFFFu && (cut == 0 || all - cut >= 8u)) {
+            if (end || (all >= need && cut <= 0xFFFFu && (cut == 0 || all - cut >= 8u))) {
                 k0 = all - need + 1u;
                 feed_points<VW, KEEP>(St, x, kind == LYON_VERB_LINE_TO, k0,
                                       ADV ? advancement_back(S, u, need - 1u)
