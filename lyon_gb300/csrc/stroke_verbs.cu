@@ -322,14 +322,14 @@ __global__ void __launch_bounds__(256) prepare_kernel(StrokeArgs A, StrokeVerbs 
     const uint32_t v0 = A.verb_offsets[0], v1 = A.verb_offsets[A.num_paths];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         S.words[0] = v1 >= v0 ? v1 - v0 : 0u;
-        if (v1 < v0) S.words[1] = 1u;
+        if (v1 < v0) S.words[1] = S.words[STROKE_VERBS_UNFIT] = 1u;
     }
     if (v1 < v0 || v1 - v0 > S.cap) return;
     for (uint32_t path = warp; path < A.num_paths; path += nwarps) {
         const uint32_t vb = A.verb_offsets[path], ve = A.verb_offsets[path + 1];
         if (ve < vb || vb < v0 || ve > v1) {
             // Not a partition of the verbs: the caller strokes the batch path by path.
-            if (lane == 0) S.words[1] = 1u;
+            if (lane == 0) S.words[1] = S.words[STROKE_VERBS_UNFIT] = 1u;
         } else if (ve - vb > 64u) {
             prepare_path<8>(A, S, path, v0, vb, ve, lane);
         } else {
@@ -1200,9 +1200,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) verb_scan_kernel(StrokeArgs A, S
     __shared__ uint32_t tile_s;
     __shared__ unsigned long long prefix_s[2];
     const uint32_t nv = batch_verbs(A);
-    // (The look-back may set words[1] while other blocks start: every thread of a block goes by one
-    // reading, and a scan that failed is not used.)
-    if (__syncthreads_or(unfit(S, nv))) return;
+    if (unfit(S, nv)) return;
     const uint32_t num_tiles = (nv + SCAN_TILE - 1) / SCAN_TILE;
     for (;;) {
         __syncthreads();

@@ -137,10 +137,10 @@ __device__ __forceinline__ uint32_t batch_verbs(const StrokeArgs& A) {
 
 // Whether the count phase has nothing to work on after prepare_kernel: more verbs than the arrays
 // hold, or offsets that run backwards (prepare_kernel does not write the slots of such a path, and
-// two paths may have written one slot, so nothing in the slots may be followed). The caller reads
-// the same words and takes the batch path by path.
+// two paths may have written one slot, so nothing in the slots may be followed). The caller takes
+// the batch path by path.
 __device__ __forceinline__ bool unfit(const StrokeVerbs& S, uint32_t verbs) {
-    return verbs > S.cap || S.words[1] != 0;
+    return verbs > S.cap || S.words[STROKE_VERBS_UNFIT] != 0;
 }
 
 }  // namespace

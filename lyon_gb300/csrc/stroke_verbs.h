@@ -36,12 +36,15 @@ struct StrokeVerbs {
     uint32_t* path_i;
     uint32_t* words;       // [0] verbs of the batch, [1] offsets out of order, [2] paths in
                            // walk_list, [3] some verb has interior steps, [4] drops, [5] scan tile,
-                           // [6] extra, [7] irregular
+                           // [6] extra, [7] irregular, [STROKE_VERBS_UNFIT] as [1], for the kernels
     unsigned long long* scan;  // tile states, after the words
     size_t clear_bytes;    // words and tile states, cleared by every count phase
 };
 constexpr uint32_t STROKE_VERBS_READ = 4;    // words the host reads back
-constexpr uint32_t STROKE_VERBS_WORDS = 16;  // words in all
+constexpr uint32_t STROKE_VERBS_WORDS = 64;  // words in all
+// A word that every warp reads, on a 128-byte line without the counters: beside them walk_kernel
+// took 66 instead of 50 us for 1,000 paths of 16 segments.
+constexpr uint32_t STROKE_VERBS_UNFIT = 32;
 // Bytes per verb of the arrays above, for their allocation.
 constexpr size_t STROKE_VERBS_BYTES = 3 * 16 + 8 + 9 * 4 + 2 + 1;
 
