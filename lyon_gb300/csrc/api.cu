@@ -470,7 +470,7 @@ const lg::SideStreams& side_streams(lyon_gpu_context* ctx) {
         ctx->side_made = true;
         int priority = 0;
         cudaStreamGetPriority(ctx->stream, &priority);
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < lg::SideStreams::N; ++i) {
             lg::SideStreams& d = ctx->side;
             if (cudaStreamCreateWithPriority(&d.stream[i], cudaStreamNonBlocking, priority) !=
                     cudaSuccess ||
@@ -624,18 +624,25 @@ int pipeline_emit(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch,
         a.indices = iout;
         if (n > 0 && tv > 0 && ctx->verbs_valid) {
             const lg::StrokeVerbs v = stroke_verbs(ctx, n);
-            if (!set_err(ctx, "stroke emit",
-                         lg::launch_stroke_verbs_emit(a, v, ctx->verb_count, ctx->verb_runs,
-                                                      ctx->num_sms, side_streams(ctx), s)))
-                return LYON_ERR_CUDA;
-            if (ctx->walk_paths > 0) {
-                a.order = v.walk_list;
-                a.item_split = v.words + 2;
-                a.list_only = 1;
-                cudaMemsetAsync(small_words(ctx), 0, 4, s);
+            const lg::SideStreams& side = side_streams(ctx);
+            const uint32_t walk = ctx->walk_paths;
+            // The paths left to the walk and the others write different parts of the output.
+            if (walk > 0) {
+                const cudaStream_t w = walk < n ? side.fork(2, s) : s;
+                lg::StrokeArgs l = a;
+                l.order = v.walk_list;
+                l.item_split = v.words + 2;
+                l.list_only = 1;
+                cudaMemsetAsync(small_words(ctx), 0, 4, w);
                 if (!set_err(ctx, "stroke emit",
-                             lg::launch_stroke(a, true, stroke_grid(ctx, ctx->walk_paths), s)))
+                             lg::launch_stroke(l, true, stroke_grid(ctx, walk), w)))
                     return LYON_ERR_CUDA;
+            }
+            if (walk < n) {
+                const cudaError_t e = lg::launch_stroke_verbs_emit(
+                    a, v, ctx->verb_count, ctx->verb_runs, ctx->num_sms, side, s);
+                if (walk > 0) side.join(2, s);
+                if (!set_err(ctx, "stroke emit", e)) return LYON_ERR_CUDA;
             }
         } else if (n > 0 && tv > 0) {
             cudaMemsetAsync(small_words(ctx), 0, 4, s);
@@ -1192,7 +1199,7 @@ void lyon_gpu_destroy(lyon_gpu_context* ctx) {
     for (int i = 0; i < 2; ++i)
         if (ctx->slot_done[i]) cudaEventDestroy(ctx->slot_done[i]);
     if (ctx->emitted) cudaEventDestroy(ctx->emitted);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < lg::SideStreams::N; ++i) {
         if (ctx->side.forked[i]) cudaEventDestroy(ctx->side.forked[i]);
         if (ctx->side.joined[i]) cudaEventDestroy(ctx->side.joined[i]);
         if (ctx->side.stream[i]) cudaStreamDestroy(ctx->side.stream[i]);

@@ -459,14 +459,28 @@ __device__ __forceinline__ void store_chain(const StrokeVerbs& S, uint32_t v, ui
     S.flags[v] = (uint16_t)f;
 }
 
+// The most steps of an irregular verb: beyond, its path is left to the walk, which takes 32 steps at a
+// time. For count and emit pass together a thread takes 1 to 2.6 us a step, the walk 0.13 us a step,
+// 3.4 us a verb of the path and, once a batch, 100 us of further launches; in a large batch the other
+// verbs take longer than that one thread. The replay that finds whether the verb can be cut instead
+// takes 0.3 us a step: it is tried for REPLAY_STEPS times as many where points merge at one cusp or
+// none (a drawn cusp; what else there is can hardly be cut). One path of one curve that turns round twice, 1,864 steps: 1266 -> 434 us,
+// by the walk 338; 2,000 paths of ten such curves of 590 steps 3527 -> 1200 us, 976.
+__device__ __forceinline__ uint32_t serial_steps(const StrokeArgs& A, uint32_t path, uint32_t nv) {
+    const uint32_t verbs = A.verb_offsets[path + 1] - A.verb_offsets[path];
+    return max(64u + verbs + verbs / 2u, nv / 500u);
+}
+constexpr uint32_t REPLAY_STEPS = 8;
+
 struct WalkSlot {
     UnitSmem u;
     float thr, hw;
     uint32_t store;  // the verb's slot when it is this one unit: its points next to the ends go
                      // straight out; else NO_STORE
-    uint32_t rough;  // some point merges, or a skip is not ruled out
+    uint32_t rough;  // some point merges
+    uint32_t skip;   // some skip is not ruled out
     uint32_t bad, badk;  // interior joins that are no flattening steps, one of them
-    uint32_t pad[2];
+    uint32_t pad;
 };
 constexpr uint32_t NO_STORE = 0xFFFFFFFFu;
 struct WalkSmem {
@@ -538,7 +552,7 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
             r.thr = thr;
             r.hw = hw;
             r.store = rb ? NO_STORE : v;
-            r.rough = r.bad = r.badk = 0;
+            r.rough = r.skip = r.bad = r.badk = 0;
         }
         __syncwarp();
         V2 q = V2{0.0f, 0.0f}, ne = V2{0.0f, 0.0f};
@@ -561,11 +575,10 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
                 ne = q - qp;
                 const V2 pe = V2{from_left(ne.x, old_e.x, lane), from_left(ne.y, old_e.y, lane)};
                 if (at < rn) {
-                    bool rough = sqlen(ne) < r.thr;
-                    // The join at this point, when it is interior: its skip test, and whether
-                    // lyon steps it as a flattened point (a parameter of exactly 1 is an end).
-                    rough |= k < m && (t == 1.0f || !skip_impossible(qp, q, ne, r.hw));
-                    if (rough) r.rough = 1u;
+                    // The join at this point, when it is interior: whether lyon steps it as a
+                    // flattened point (a parameter of exactly 1 is an end), and its skip test.
+                    if (sqlen(ne) < r.thr || (k < m && t == 1.0f)) r.rough = 1u;
+                    if (k < m && !skip_impossible(qp, q, ne, r.hw)) r.skip = 1u;
                     // The join at the point before.
                     if (k > 1u && !(dot(pe, ne) > 0.0f)) {
                         atomicAdd(&r.bad, 1u);
@@ -583,15 +596,22 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
         }
         if (ra) {
             const WalkSlot& x = sm.unit[slot];
-            uint32_t rough = x.rough, bad = x.bad, badk = x.badk;
+            uint32_t rough = x.rough, skip = x.skip, bad = x.bad, badk = x.badk;
             if (rb) {
                 rough |= sm.unit[slot + 1].rough;
+                skip |= sm.unit[slot + 1].skip;
                 bad += sm.unit[slot + 1].bad;
             }
             // One cusp cuts the verb in two runs, unless it is split already. (A clipped miter there
             // leaves sides that are not symmetric, as the skip test's bound wants them:
             // extra_count_kernel evaluates the test at the join after it.)
-            if (rough || bad > 1 || (bad == 1 && rb)) {
+            const bool irregular = rough || skip || bad > 1 || (bad == 1 && rb);
+            // (The walk of a variable-width path is one thread's as well.)
+            const uint32_t most = irregular && !A.widths ? serial_steps(A, path, nv) : steps;
+            const bool refused = skip && !rough && bad == 0 && !rb;  // walk_irregular comes to that
+            if ((refused && !A.widths) || steps > (rough && bad <= 1 && !rb ? REPLAY_STEPS * most : most)) {
+                leave_to_walk(S, path);
+            } else if (irregular) {
                 Chain c;
                 replay_chain(a, b, c1, thr, hw, c);
                 if (c.cuttable) {
@@ -600,6 +620,8 @@ __global__ void __launch_bounds__(WIN_WARPS * 32) walk_kernel(StrokeArgs A, Stro
                     S.cut[v] = c.at | (c.gap << 16);
                     S.extra[atomicAdd(&S.words[6], 1u)] = v;
                     if (a.m > c.gap + 2u) S.words[3] = 1u;
+                } else if (steps > most) {
+                    leave_to_walk(S, path);
                 } else {
                     store_chain(S, v, path, VF_IRR | (flags & VF_TURN), c);
                     if (!c.end_kept) S.drops[atomicAdd(&S.words[4], 1u)] = v;

@@ -52,8 +52,9 @@ constexpr size_t STROKE_VERBS_BYTES = 3 * 16 + 8 + 9 * 4 + 2 + 1;
 // that continues after what is on `s`, join(i, s) makes `s` wait for it. Without streams (none
 // could be made) the work goes on `s` itself.
 struct SideStreams {
-    cudaStream_t stream[2] = {nullptr, nullptr};
-    cudaEvent_t forked[2] = {nullptr, nullptr}, joined[2] = {nullptr, nullptr};
+    static constexpr int N = 3;
+    cudaStream_t stream[N] = {};
+    cudaEvent_t forked[N] = {}, joined[N] = {};
     cudaStream_t fork(int i, cudaStream_t s) const {
         if (!stream[i]) return s;
         cudaEventRecord(forked[i], s);
