@@ -135,6 +135,12 @@ __device__ __forceinline__ uint32_t batch_verbs(const StrokeArgs& A) {
     return b >= a ? b - a : 0u;
 }
 
+// Slots per tile of a grid whose blocks take tiles in turn: `most`, or fewer (at least `least`) when
+// that would leave blocks without a tile.
+__device__ __forceinline__ uint32_t tile_size(uint32_t nv, uint32_t least, uint32_t most) {
+    return min(most, max(least, (nv + gridDim.x - 1u) / gridDim.x));
+}
+
 // Whether the count phase has nothing to work on after prepare_kernel: more verbs than the arrays
 // hold, or offsets that run backwards (prepare_kernel does not write the slots of such a path, and
 // two paths may have written one slot, so nothing in the slots may be followed). The caller takes
