@@ -632,29 +632,42 @@ __device__ __forceinline__ void step_verb(const StrokeArgs& A, const StrokeVerbs
     }
 }
 
-// Threads take the verbs of a tile sorted by what they are (curves, lines, ends), so that the
-// lanes of a warp do much the same.
-constexpr uint32_t STEP_TILE = 512;
+// Threads take the verbs of a tile sorted by what they are (curves, lines, ends; each from a warp's
+// boundary), so that the lanes of a warp do much the same. In full tiles the kinds follow one another,
+// so that a block's warps share their instructions (10,001 curve paths of variable width 6.8 ms, with
+// the kinds side by side 7.1). A batch too small for a full tile per block has smaller tiles, with
+// the kinds side by side: 100 lines of four points and variable width 343 -> 173 us.
+constexpr uint32_t STEP_TILE = 512, STEP_TILE_LEAST = 32;
 template <bool EMIT, bool VW, class SK>
 __global__ void __launch_bounds__(128) steps_kernel(StrokeArgs A, StrokeVerbs S) {
-    __shared__ uint16_t list[STEP_TILE];
+    __shared__ uint16_t list[3][STEP_TILE];
     __shared__ uint32_t count[3];
     const uint32_t nv = batch_verbs(A);
     if (unfit(S, nv)) return;
-    for (uint32_t tile = blockIdx.x * STEP_TILE; tile < nv; tile += gridDim.x * STEP_TILE) {
-        for (int kind = 0; kind < 3; ++kind) {
-            __syncthreads();
-            if (threadIdx.x == 0) count[kind] = 0;
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < STEP_TILE && tile + i < nv; i += blockDim.x) {
-                const int k = S.kind[tile + i] & KIND_MASK;
-                const bool mine = kind == 0 ? is_segment(k) && k != LYON_VERB_LINE_TO
-                                : kind == 1 ? k == LYON_VERB_LINE_TO : is_end(k);
-                if (mine) list[atomicAdd(&count[kind], 1u)] = (uint16_t)i;
+    const uint32_t size = tile_size(nv, STEP_TILE_LEAST, STEP_TILE);
+    for (uint32_t tile = blockIdx.x * size; tile < nv; tile += gridDim.x * size) {
+        __syncthreads();
+        if (threadIdx.x < 3) count[threadIdx.x] = 0;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < size && tile + i < nv; i += blockDim.x) {
+            const int k = S.kind[tile + i] & KIND_MASK;
+            const int l = k == LYON_VERB_LINE_TO ? 1 : is_segment(k) ? 0 : is_end(k) ? 2 : 3;
+            if (l < 3) list[l][atomicAdd(&count[l], 1u)] = (uint16_t)i;
+        }
+        __syncthreads();
+        const uint32_t n0 = count[0], n1 = count[1], n2 = count[2];
+        const uint32_t s1 = (n0 + 31u) & ~31u, s2 = s1 + ((n1 + 31u) & ~31u);
+        const bool apart = size == STEP_TILE;
+        for (int pass = 0; pass < (apart ? 3 : 1); ++pass) {
+            const uint32_t from = pass == 0 ? 0u : pass == 1 ? s1 : s2;
+            const uint32_t to = !apart || pass == 2 ? s2 + n2 : pass == 0 ? s1 : s2;
+            for (uint32_t i = from + threadIdx.x; i < to; i += blockDim.x) {
+                const int l = i < s1 ? 0 : i < s2 ? 1 : 2;
+                const uint32_t j = l == 0 ? i : l == 1 ? i - s1 : i - s2;
+                if (j < (l == 0 ? n0 : l == 1 ? n1 : n2))
+                    step_verb<EMIT, VW, SK>(A, S, tile + list[l][j]);
             }
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < count[kind]; i += blockDim.x)
-                step_verb<EMIT, VW, SK>(A, S, tile + list[i]);
+            if (apart) __syncthreads();
         }
     }
 }
