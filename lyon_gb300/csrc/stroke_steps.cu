@@ -143,8 +143,14 @@ __device__ __forceinline__ float running_sums(const float4* lengths, float4* sum
     return adv;
 }
 
-// Paths of more verbs than this are taken by blocks (below), the others by warps.
+// Paths of more verbs than this are taken by blocks (below), the others by warps; so are long ones
+// that are nearly all lines (a point a verb, or fewer): a warp takes 32 lines at once.
 constexpr uint32_t ADVANCE_LONG = 64;
+__device__ __forceinline__ bool advance_by_block(const StrokeArgs& A, uint32_t path,
+                                                 uint32_t verbs) {
+    const uint32_t points = A.point_offsets[path + 1] - A.point_offsets[path];
+    return verbs > ADVANCE_LONG && points > verbs + verbs / 16u;
+}
 
 // The advancement at edge e's end, of M, where it is one of the last four; with `first` (the edges of
 // the first of two runs) the one between the runs takes the first place.
@@ -169,15 +175,35 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
     const bool runs = !A.widths && !A.sources;  // records: written run by run (stroke_verbs.cu)
     for (uint32_t path = warp; path < A.num_paths; path += nwarps) {
         const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
-        if (s1 - s0 > ADVANCE_LONG || S.path_walk[path]) continue;
+        if (advance_by_block(A, path, s1 - s0) || S.path_walk[path]) continue;
         const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
         AdvanceState st{0.0f, 0.0f, 0};
         for (uint32_t base = s0; base < s1; base += 32) {
             const uint32_t n = min(32u, s1 - base);
             const int kind = (uint32_t)lane < n ? S.kind[base + lane] & KIND_MASK : KIND_NONE;
+            const uint32_t lines = __ballot_sync(FULL, kind == LYON_VERB_LINE_TO);
             for (uint32_t i = 0; i < n; ++i) {
                 const uint32_t v = base + i;
                 const int k = __shfl_sync(FULL, kind, (int)i);
+                // Lines in a row: lane = verb.
+                const uint32_t others = ~lines >> i;
+                const uint32_t row = others ? (uint32_t)__ffs((int)others) - 1u : 32u - i;
+                if (row > 1u) {
+                    const uint32_t u = v + (uint32_t)lane;
+                    float len = 0.0f;
+                    if ((uint32_t)lane < row)
+                        len = vlength(end_point(S, A.points, u) - last_kept(S, A.points, u - 1));
+                    reinterpret_cast<float*>(len4)[lane] = len;
+                    __syncwarp();
+                    st.adv = running_sums(len4, sum4, (row + 3u) / 4u, st.adv, lane);
+                    __syncwarp();
+                    if ((uint32_t)lane < row)
+                        out[4 * (size_t)u + 3] = reinterpret_cast<const float*>(sum4)[lane];
+                    __syncwarp();
+                    st.kept += row;
+                    i += row - 1u;
+                    continue;
+                }
                 if (!is_segment(k) || (S.flags[v] & VF_IRR)) {
                     advance_special(A, S, v, k, P, st, lane);
                     continue;
@@ -206,111 +232,125 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
     __shared__ uint32_t first[33];
     __shared__ int kinds[32];
     __shared__ uint32_t split[32];  // edges of the first of two runs, else 0
-    __shared__ uint32_t window;
+    __shared__ uint32_t window, num_long;
+    __shared__ uint16_t longs[256];
     float* len = reinterpret_cast<float*>(room);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (unfit(S, batch_verbs(A))) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
     const bool runs = !A.widths && !A.sources;
-    for (uint32_t path = blockIdx.x; path < A.num_paths; path += gridDim.x) {
-        const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
-        if (s1 - s0 <= ADVANCE_LONG || S.path_walk[path]) continue;
-        const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
-        AdvanceState st{0.0f, 0.0f, 0};
-        for (uint32_t base = s0; base < s1;) {
-            __syncthreads();
-            if (warp == 0) {
-                // The window's verbs, their points rounded up to 16-byte words.
-                const uint32_t v = base + (uint32_t)lane;
-                int k = v < s1 ? S.kind[v] & KIND_MASK : KIND_NONE;
-                uint32_t m = 0, m1 = 0;
-                if (is_segment(k)) {
-                    const uint32_t flags = S.flags[v];
-                    if (flags & VF_IRR) {
-                        k |= 8;
-                    } else {
-                        Unit a, b;
-                        verb_units(k, S.rec[v], A.points, P.tolerance, flags,
-                                   flags & VF_TWO ? S.cut[v] : 0u, a, b);
-                        m = a.m + b.m;
-                        if (runs && b.m) m1 = a.m;
+    // A block looks through a tile of paths at once, and takes the long ones.
+    const uint32_t size = tile_size(A.num_paths, 1u, 256u);
+    for (uint32_t tile = blockIdx.x * size; tile < A.num_paths; tile += gridDim.x * size) {
+        __syncthreads();
+        if (threadIdx.x == 0) num_long = 0;
+        __syncthreads();
+        if (threadIdx.x < size && tile + threadIdx.x < A.num_paths) {
+            const uint32_t p = tile + threadIdx.x;
+            if (advance_by_block(A, p, A.verb_offsets[p + 1] - A.verb_offsets[p]) && !S.path_walk[p])
+                longs[atomicAdd(&num_long, 1u)] = (uint16_t)threadIdx.x;
+        }
+        __syncthreads();
+        for (uint32_t at = 0; at < num_long; ++at) {
+            const uint32_t path = tile + longs[at];
+            const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
+            const StrokeParams P = make_params(A.options[A.num_options > 1 ? path : 0]);
+            AdvanceState st{0.0f, 0.0f, 0};
+            for (uint32_t base = s0; base < s1;) {
+                __syncthreads();
+                if (warp == 0) {
+                    // The window's verbs, their points rounded up to 16-byte words.
+                    const uint32_t v = base + (uint32_t)lane;
+                    int k = v < s1 ? S.kind[v] & KIND_MASK : KIND_NONE;
+                    uint32_t m = 0, m1 = 0;
+                    if (is_segment(k)) {
+                        const uint32_t flags = S.flags[v];
+                        if (flags & VF_IRR) {
+                            k |= 8;
+                        } else {
+                            Unit a, b;
+                            verb_units(k, S.rec[v], A.points, P.tolerance, flags,
+                                       flags & VF_TWO ? S.cut[v] : 0u, a, b);
+                            m = a.m + b.m;
+                            if (runs && b.m) m1 = a.m;
+                        }
                     }
-                }
-                split[lane] = m1;
-                uint32_t incl = (m + 3u) & ~3u;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t up = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o) incl += up;
-                }
-                first[lane] = incl - ((m + 3u) & ~3u);
-                kinds[lane] = k | (int)(m << 4);
-                const uint32_t fit = __ballot_sync(FULL, incl <= ADVANCE_ROOM && v < s1);
-                if (lane == 0) window = (uint32_t)__popc(fit);
-            }
-            __syncthreads();
-            const uint32_t n = window;
-            for (uint32_t i = (uint32_t)warp; i < n; i += blockDim.x / 32) {
-                const int k = kinds[i] & 15;
-                if (!is_segment(k)) continue;
-                verb_edges(A, S, base + i, k, P, lane,
-                           [&](uint32_t e, uint32_t, float x, uint32_t M, uint32_t) {
-                               if (e < M) len[first[i] + e] = x;
-                           });
-                const uint32_t m = (uint32_t)kinds[i] >> 4;  // (zeros up to the word's end)
-                if (m + (uint32_t)lane < ((m + 3u) & ~3u)) len[first[i] + m + lane] = 0.0f;
-            }
-            __syncthreads();
-            if (warp == 0 && n == 0) {
-                // One verb of more points than there is room for.
-                const int k = kinds[0] & 15;
-                st.kept += verb_edges(A, S, base, k, P, lane, [&](uint32_t e, uint32_t cnt, float x,
-                                                                  uint32_t M, uint32_t m1) {
-                    float mine = 0.0f;
-                    for (uint32_t j = 0; j < cnt; ++j) {
-                        st.adv = st.adv + __shfl_sync(FULL, x, (int)j);
-                        if ((uint32_t)lane == j) mine = st.adv;
+                    split[lane] = m1;
+                    uint32_t incl = (m + 3u) & ~3u;
+    #pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t up = __shfl_up_sync(FULL, incl, o);
+                        if (lane >= o) incl += up;
                     }
-                    keep_advancement(out + 4 * (size_t)base, e, M, runs ? m1 : 0u, mine);
-                });
-            }
-            // The sums of the window's rows of run verbs; lane = verb then takes its four.
-            const int mine = warp == 0 && (uint32_t)lane < n ? kinds[lane] : KIND_NONE;
-            const uint32_t special = __ballot_sync(FULL, !is_segment(mine & 15));
-            for (uint32_t i = 0; warp == 0 && i < n;) {
-                if ((special >> i) & 1u) {
-                    advance_special(A, S, base + i, (kinds[i] & 15) & 7, P, st, lane);
-                    ++i;
-                    continue;
+                    first[lane] = incl - ((m + 3u) & ~3u);
+                    kinds[lane] = k | (int)(m << 4);
+                    const uint32_t fit = __ballot_sync(FULL, incl <= ADVANCE_ROOM && v < s1);
+                    if (lane == 0) window = (uint32_t)__popc(fit);
                 }
-                const uint32_t rest = special >> i;
-                const uint32_t end = rest ? min(n, i + (uint32_t)__ffs((int)rest) - 1u) : n;
-                const uint32_t w0 = first[i] / 4u;
-                const uint32_t w1 = (first[end - 1u] + ((uint32_t)kinds[end - 1u] >> 4) + 3u) / 4u;
-                const float start = st.adv;
-                st.adv = running_sums(room + w0, sums + w0, w1 - w0, start, lane);
-                __syncwarp();
-                const float* sum = reinterpret_cast<const float*>(sums);
-                uint32_t m = 0;
-                if ((uint32_t)lane >= i && (uint32_t)lane < end) {
-                    m = (uint32_t)mine >> 4;
-                    const uint32_t f = first[lane], m1 = split[lane];
-                    const float before =
-                        (uint32_t)lane == i ? start
-                                            : sum[first[lane - 1] + ((uint32_t)kinds[lane - 1] >> 4) - 1u];
-                    float a[4];
-#pragma unroll
-                    for (uint32_t c = 0; c < 4; ++c)
-                        a[c] = m + c >= 4u ? sum[f + m + c - 4u] : m + c == 3u ? before : 0.0f;
-                    if (m1) a[0] = sum[f + m1 - 1u];
-                    advancements(S)[base + lane] = make_float4(a[0], a[1], a[2], a[3]);
+                __syncthreads();
+                const uint32_t n = window;
+                for (uint32_t i = (uint32_t)warp; i < n; i += blockDim.x / 32) {
+                    const int k = kinds[i] & 15;
+                    if (!is_segment(k)) continue;
+                    verb_edges(A, S, base + i, k, P, lane,
+                               [&](uint32_t e, uint32_t, float x, uint32_t M, uint32_t) {
+                                   if (e < M) len[first[i] + e] = x;
+                               });
+                    const uint32_t m = (uint32_t)kinds[i] >> 4;  // (zeros up to the word's end)
+                    if (m + (uint32_t)lane < ((m + 3u) & ~3u)) len[first[i] + m + lane] = 0.0f;
                 }
-                st.kept += __reduce_add_sync(FULL, m);
-                __syncwarp();
-                i = end;
+                __syncthreads();
+                if (warp == 0 && n == 0) {
+                    // One verb of more points than there is room for.
+                    const int k = kinds[0] & 15;
+                    st.kept += verb_edges(A, S, base, k, P, lane, [&](uint32_t e, uint32_t cnt, float x,
+                                                                      uint32_t M, uint32_t m1) {
+                        float mine = 0.0f;
+                        for (uint32_t j = 0; j < cnt; ++j) {
+                            st.adv = st.adv + __shfl_sync(FULL, x, (int)j);
+                            if ((uint32_t)lane == j) mine = st.adv;
+                        }
+                        keep_advancement(out + 4 * (size_t)base, e, M, runs ? m1 : 0u, mine);
+                    });
+                }
+                // The sums of the window's rows of run verbs; lane = verb then takes its four.
+                const int mine = warp == 0 && (uint32_t)lane < n ? kinds[lane] : KIND_NONE;
+                const uint32_t special = __ballot_sync(FULL, !is_segment(mine & 15));
+                for (uint32_t i = 0; warp == 0 && i < n;) {
+                    if ((special >> i) & 1u) {
+                        advance_special(A, S, base + i, (kinds[i] & 15) & 7, P, st, lane);
+                        ++i;
+                        continue;
+                    }
+                    const uint32_t rest = special >> i;
+                    const uint32_t end = rest ? min(n, i + (uint32_t)__ffs((int)rest) - 1u) : n;
+                    const uint32_t w0 = first[i] / 4u;
+                    const uint32_t w1 = (first[end - 1u] + ((uint32_t)kinds[end - 1u] >> 4) + 3u) / 4u;
+                    const float start = st.adv;
+                    st.adv = running_sums(room + w0, sums + w0, w1 - w0, start, lane);
+                    __syncwarp();
+                    const float* sum = reinterpret_cast<const float*>(sums);
+                    uint32_t m = 0;
+                    if ((uint32_t)lane >= i && (uint32_t)lane < end) {
+                        m = (uint32_t)mine >> 4;
+                        const uint32_t f = first[lane], m1 = split[lane];
+                        const float before =
+                            (uint32_t)lane == i ? start
+                                                : sum[first[lane - 1] + ((uint32_t)kinds[lane - 1] >> 4) - 1u];
+                        float a[4];
+    #pragma unroll
+                        for (uint32_t c = 0; c < 4; ++c)
+                            a[c] = m + c >= 4u ? sum[f + m + c - 4u] : m + c == 3u ? before : 0.0f;
+                        if (m1) a[0] = sum[f + m1 - 1u];
+                        advancements(S)[base + lane] = make_float4(a[0], a[1], a[2], a[3]);
+                    }
+                    st.kept += __reduce_add_sync(FULL, m);
+                    __syncwarp();
+                    i = end;
+                }
+                base += n > 0 ? n : 1u;
             }
-            base += n > 0 ? n : 1u;
         }
     }
 }
