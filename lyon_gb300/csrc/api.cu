@@ -52,7 +52,7 @@ struct lyon_gpu_context {
     // per-path work arrays
     DevBuf vtx_counts, idx_counts, status, vtx_offsets, idx_offsets, scan_state;
     DevBuf small;  // [0] work counter, [1] scan counter, [2] error flag, [3] failed paths,
-                   // [4..5] processing-order counters
+                   // [4..5] processing-order counters, [6] short paths, [8..10] batch shape
     DevBuf order;  // processing order of the current stroke batch (long paths first)
     // lyon_gpu_svg_parse_paths: counts, diagnostics, offsets and the parsed batch.
     DevBuf svg_counts, svg_diag, svg_off64, svg_off32, svg_verbs, svg_points, svg_widths;
@@ -66,6 +66,7 @@ struct lyon_gpu_context {
     uint32_t verb_cap = 0;      // verbs verb_mem holds
     uint32_t verb_count = 0;    // verbs of the last counted batch
     uint32_t verbs_known = 0;   // the coming batch's verbs when the caller knows them, else 0
+    uint32_t points_known = 0;  // and the points of a batch of one path, when verbs_known is set
     bool verbs_valid = false;   // the last count phase was verb-parallel
     bool verb_runs = false;     // its batch has curves with interior steps
     uint32_t walk_paths = 0;    // its paths left to the walk
@@ -485,16 +486,77 @@ const lg::SideStreams& side_streams(lyon_gpu_context* ctx) {
     return ctx->side;
 }
 
+// Whether a batch of this shape is stroked sooner path by path (by the walk, its short line-only paths
+// by a thread each, or with widths and sources by the stepper, a thread per path) than verb by verb:
+// many short paths fill the GPU by themselves, and the passes over the verbs and the steps before
+// each verb come on top. Microseconds path by path and verb by verb:
+//   positions, lines of two points: 10,000 121 and 127, 100,000 163 and 255, 400,000 372 and 733; of
+//     eight points 236 and 143, 400 and 398, 1157 and 1315; of 16, 100,000: 714 and 538.
+//   records, lines of two points: 10,000 122 and 138, 100,000 170 and 347; of eight, 426 and 523; of
+//     16, 772 and 696.
+//   sources, lines of four points: 10,000 150 and 176, 100,000 236 and 587; of 32, 10,000 662 and
+//     444, 100,000 1269 and 3410. (Curves: verb by verb from one path on.)
+//   widths, lines of four points: 1 106 and 169, 1,000 126 and 193, 10,000 199 and 346, 100,000 304
+//     and 1630; of 32, 1,000 760 and 284, 10,000 1095 and 1427, 100,000 2024 and 11898; two cubics:
+//     100 444 and 309, 10,000 878 and 1003, 100,000 1548 and 4184; 16: 10,000 6260 and 2887.
+// For widths that is a thread's 30 us a step of the longest path against 3.9 ns a line's step and 1.4
+// ns a curve's, and 250 us; for sources 20 us against 1.03 ns. A curve has about 14 steps, for the two
+// points of it (a quadratic: one) that its path has more than verbs.
+constexpr uint32_t LINES_BY_PATH = 32768, RECORDS_BY_PATH = 16384;  // paths
+constexpr uint32_t SHORT_LINES = 32;                                // points
+bool by_path_sooner(const lyon_gpu_context* ctx, uint32_t n, const lg::BatchShape& b) {
+    const bool lines = b.points <= b.verbs + b.verbs / 16;
+    auto steps = [](uint32_t verbs, uint32_t points) {
+        return verbs + (points > verbs ? 6.5 * (points - verbs) : 0.0);
+    };
+    if (ctx->vw_widths)
+        return 30.0 * steps(b.max_verbs, b.max_points) <
+               (lines ? 0.0039 : 0.0014) * steps(b.verbs, b.points) + 250.0;
+    if (!lines) return false;
+    if (ctx->want_sources) return n >= RECORDS_BY_PATH && 20.0 * b.max_verbs < 0.00103 * b.verbs;
+    if (b.max_points > SHORT_LINES) return false;
+    if (ctx->vertex_attrs) return n >= RECORDS_BY_PATH && b.points <= 10.0 * n;
+    return n >= LINES_BY_PATH && b.points <= 8.5 * n;
+}
+// Whether by_path_sooner can hold at all for so many paths: only then is the shape asked for.
+bool may_be_sooner(const lyon_gpu_context* ctx, uint32_t n) {
+    return ctx->vw_widths ? true
+           : n >= (ctx->want_sources || ctx->vertex_attrs ? RECORDS_BY_PATH : LINES_BY_PATH);
+}
+
+// The shape of a batch of the device's (one wait for the stream).
+bool batch_shape(lyon_gpu_context* ctx, const lyon_path_batch* batch, lg::BatchShape* out) {
+    if (batch->num_paths == 1 && ctx->verbs_known) {
+        *out = lg::BatchShape{ctx->verbs_known, ctx->points_known, ctx->verbs_known,
+                              ctx->points_known};
+        return true;
+    }
+    if (!ensure_host(ctx, ctx->h_small, 64)) return false;
+    cudaStream_t s = ctx->stream;
+    uint32_t* words = small_words(ctx) + 8;  // three for the maxima, then the shape
+    lg::BatchShape* host = reinterpret_cast<lg::BatchShape*>(ctx->h_small.ptr);
+    lg::BatchShape* mapped = direct_host_pointer<lg::BatchShape>(host);
+    lg::BatchShape* dev = mapped ? mapped : reinterpret_cast<lg::BatchShape*>(words + 4);
+    if (!set_err(ctx, "batch shape",
+                 lg::launch_batch_shape(batch->verb_offsets, batch->point_offsets,
+                                        batch->num_paths, words, dev, ctx->num_sms, s)))
+        return false;
+    if (!mapped) cudaMemcpyAsync(host, dev, sizeof *host, cudaMemcpyDeviceToHost, s);
+    if (!set_err(ctx, "sync", cudaStreamSynchronize(s))) return false;
+    *out = *host;
+    return true;
+}
+
 // Counts a stroke verb by verb. Returns LYON_OK with ctx->verbs_valid
 // false when the batch is left to the path-by-path count (its offsets overlap, or no room for the
 // arrays).
+// `need`: the batch's verbs, 0 when they are not known.
 int count_by_verb(lyon_gpu_context* ctx, const lyon_path_batch* batch,
                   const lyon_stroke_options* options, uint32_t num_options, int index_bits,
-                  int index_mode, uint64_t vertex_offset, uint64_t* tv, uint64_t* ti,
-                  uint32_t* failed) {
+                  int index_mode, uint64_t vertex_offset, uint32_t need, uint64_t* tv,
+                  uint64_t* ti, uint32_t* failed) {
     const uint32_t n = batch->num_paths;
     cudaStream_t s = ctx->stream;
-    uint32_t need = ctx->verbs_known;
     if (need == 0 && ctx->verb_cap == 0) {
         // The first batch: its size is on the device. Later ones are tried with the arrays there
         // are, and counted again when they hold more.
@@ -554,9 +616,18 @@ int pipeline_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch
     ctx->order_valid = false;
     ctx->split_valid = false;
     ctx->verbs_valid = false;
-    if (kind == KIND_STROKE && n > 0) {
+    uint32_t verbs = ctx->verbs_known;
+    bool by_path = kind != KIND_STROKE || n == 0;
+    if (!by_path && may_be_sooner(ctx, n)) {
+        lg::BatchShape shape;
+        if (!batch_shape(ctx, batch, &shape)) return LYON_ERR_CUDA;
+        verbs = shape.verbs;
+        // (A path with more verbs than the batch: offsets that run backwards.)
+        by_path = shape.max_verbs > shape.verbs || by_path_sooner(ctx, n, shape);
+    }
+    if (!by_path) {
         const int r = count_by_verb(ctx, batch, (const lyon_stroke_options*)options, num_options,
-                                    index_bits, index_mode, vertex_offset, tv, ti, failed);
+                                    index_bits, index_mode, vertex_offset, verbs, tv, ti, failed);
         if (r != LYON_OK) return r;
         if (ctx->verbs_valid) {
             mark(ctx, 2);
@@ -949,6 +1020,7 @@ int single_path(lyon_gpu_context* ctx, int kind, const uint8_t* verbs, uint32_t 
     }
     lyon_gpu_batch_output bo;
     ctx->verbs_known = num_verbs;
+    ctx->points_known = num_points;
     int r = batched_device(ctx, kind, &b, ctx->in_options.ptr, 1, index_bits,
                            LYON_INDEX_PER_PATH, index_base, &bo);
     ctx->verbs_known = 0;

@@ -169,6 +169,15 @@ cudaError_t launch_read_totals(const uint64_t* a_total, const uint64_t* b_total,
                                const uint32_t* words, const uint32_t* more, uint64_t* host_dst,
                                cudaStream_t s);
 
+// What a batch's offsets say of it: its verbs and points, and the most of each that a path has.
+struct BatchShape {
+    uint32_t verbs, points, max_verbs, max_points;
+};
+// Into *out (device memory, or mapped host memory). `work`: three words, cleared here.
+cudaError_t launch_batch_shape(const uint32_t* verb_offsets, const uint32_t* point_offsets,
+                               uint32_t n, uint32_t* work, BatchShape* out, int num_sms,
+                               cudaStream_t s);
+
 // Processing order by class: paths with more than `big_points` points (0: none) first, then the
 // other paths, then line-only paths of at most `short_points` points (0: none; at most
 // CLASSIFY_MAX_SHORT_POINTS) by decreasing point count: the one-thread-per-path phase of the

@@ -204,6 +204,45 @@ __global__ void classify_place_kernel(const uint8_t* path_class, uint32_t n,
     if (i < n) order[start[c] + local[c] + rank] = i;
 }
 
+__global__ void __launch_bounds__(256)
+    batch_shape_kernel(const uint32_t* verb_offsets, const uint32_t* point_offsets, uint32_t n,
+                       uint32_t* work, BatchShape* out) {
+    __shared__ uint32_t most[2];
+    if (threadIdx.x < 2) most[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t v = 0, p = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        v = max(v, verb_offsets[i + 1] - verb_offsets[i]);
+        p = max(p, point_offsets[i + 1] - point_offsets[i]);
+    }
+    v = __reduce_max_sync(0xFFFFFFFFu, v);
+    p = __reduce_max_sync(0xFFFFFFFFu, p);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&most[0], v);
+        atomicMax(&most[1], p);
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    atomicMax(&work[0], most[0]);
+    atomicMax(&work[1], most[1]);
+    __threadfence();
+    if (atomicAdd(&work[2], 1u) + 1u < gridDim.x) return;
+    __threadfence();  // the last block: the others' maxima are there
+    *out = BatchShape{verb_offsets[n] - verb_offsets[0], point_offsets[n] - point_offsets[0],
+                      atomicMax(&work[0], 0u), atomicMax(&work[1], 0u)};
+}
+
+cudaError_t launch_batch_shape(const uint32_t* verb_offsets, const uint32_t* point_offsets,
+                               uint32_t n, uint32_t* work, BatchShape* out, int num_sms,
+                               cudaStream_t s) {
+    cudaMemsetAsync(work, 0, 12, s);
+    const uint32_t need = (n + 1023) / 1024, most = 4u * (uint32_t)(num_sms > 0 ? num_sms : 1);
+    batch_shape_kernel<<<need < 1 ? 1 : need < most ? need : most, 256, 0, s>>>(
+        verb_offsets, point_offsets, n, work, out);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
 // Order by size: bin 31 - floor(log2(points)) (0 points: bin 32), so bigger paths come first.
 __global__ void size_count_kernel(const uint32_t* point_offsets, const uint32_t* sizes,
                                   uint32_t n, uint8_t* cls, uint32_t* counters) {
