@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128) advance_kernel(StrokeArgs A, StrokeVerbs 
     if (unfit(S, batch_verbs(A))) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
-    const bool runs = !A.widths && !A.sources;  // records: written run by run (stroke_verbs.cu)
+    const bool runs = !A.widths && !A.sequential;  // records: written run by run (stroke_verbs.cu)
     for (uint32_t path = warp; path < A.num_paths; path += nwarps) {
         const uint32_t s0 = A.verb_offsets[path] - v0, s1 = A.verb_offsets[path + 1] - v0;
         if (advance_by_block(A, path, s1 - s0) || S.path_walk[path]) continue;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
     if (unfit(S, batch_verbs(A))) return;
     const uint32_t v0 = A.verb_offsets[0];
     float* out = reinterpret_cast<float*>(advancements(S));
-    const bool runs = !A.widths && !A.sources;
+    const bool runs = !A.widths && !A.sequential;
     // A block looks through a tile of paths at once, and takes the long ones.
     const uint32_t size = tile_size(A.num_paths, 1u, 256u);
     for (uint32_t tile = blockIdx.x * size; tile < A.num_paths; tile += gridDim.x * size) {
@@ -733,20 +733,25 @@ uint32_t blocks_for(uint32_t items, uint32_t per_block, int num_sms, uint32_t wa
 
 }  // namespace
 
-// Side by side: the long paths are few blocks, each bound by its chain of additions (20,000 paths with
-// records: 0.74 and 0.62 ms one after the other).
+// On two side streams, which the caller joins: the long paths are few blocks, each bound by its chain
+// of additions (20,000 paths with records: 0.74 and 0.62 ms one after the other). They read what
+// drops_kernel leaves.
 void launch_stroke_advance(const StrokeArgs& a, const StrokeVerbs& v, int num_sms,
                            const SideStreams& side, cudaStream_t s) {
-    const cudaStream_t l = side.fork(0, s);
+    const cudaStream_t w = side.fork(1, s), l = side.fork(2, s);
     advance_long_kernel<<<blocks_for(a.num_paths, 1, num_sms, 8), 256, 0, l>>>(a, v);
-    advance_kernel<<<blocks_for(a.num_paths, 4, num_sms, 16), 128, 0, s>>>(a, v);
-    side.join(0, s);
+    advance_kernel<<<blocks_for(a.num_paths, 4, num_sms, 16), 128, 0, w>>>(a, v);
     note_launches(2);
+}
+void join_stroke_advance(const SideStreams& side, cudaStream_t s) {
+    side.join(1, s);
+    side.join(2, s);
 }
 
 void launch_stroke_steps_count(const StrokeArgs& a, const StrokeVerbs& v, uint32_t verbs_hint,
                                int num_sms, const SideStreams& side, cudaStream_t s) {
     launch_stroke_advance(a, v, num_sms, side, s);
+    join_stroke_advance(side, s);
     steps_kernel<false, true, Sink>
         <<<blocks_for(verbs_hint, STEP_TILE, num_sms, 16), 128, 0, s>>>(a, v);
     check_states_kernel<<<blocks_for(verbs_hint, 256, num_sms, 8), 256, 0, s>>>(a, v);
@@ -769,7 +774,10 @@ cudaError_t launch_stroke_steps_emit(const StrokeArgs& a, const StrokeVerbs& v,
         }
     } else {
         if (a.vertex_attrs) {
-            launch_stroke_advance(a, v, num_sms, side, s);
+            if (a.num_paths > STROKE_ADVANCE_EARLY) {
+                launch_stroke_advance(a, v, num_sms, side, s);
+                join_stroke_advance(side, s);
+            }
             steps_kernel<true, false, SrcSinkT<true>><<<grid, 128, 0, s>>>(a, v);
         } else {
             steps_kernel<true, false, SrcSinkT<false>><<<grid, 128, 0, s>>>(a, v);

@@ -1702,6 +1702,8 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
     walk_kernel<<<grid_for(verbs_hint, WIN_WARPS, num_sms, 8), WIN_WARPS * 32,
                   WIN_WARPS * sizeof(WalkSmem), s>>>(a, v);
     drops_kernel<<<grid_for(0, 128, num_sms, 1), 128, 0, s>>>(a, v);
+    const bool advance = a.vertex_attrs && !a.widths && n <= STROKE_ADVANCE_EARLY;
+    if (advance) launch_stroke_advance(a, v, num_sms, side, s);
     if (a.widths) {
         launch_stroke_steps_count(a, v, verbs_hint, num_sms, side, s);
     } else {
@@ -1718,15 +1720,16 @@ cudaError_t launch_stroke_verbs_count(const StrokeArgs& a, const StrokeVerbs& v,
     const bool one_tile = finish && verbs_hint <= SCAN_TILE;
     if (one_tile) {
         finish_kernel<true><<<1, SCAN_THREADS, 0, s>>>(a, v, *finish);
-        return cudaGetLastError();
-    }
-    verb_scan_kernel<<<grid_for(verbs_hint, SCAN_TILE, num_sms, 4), SCAN_THREADS, 0, s>>>(a, v);
-    if (finish) {
-        finish_kernel<false><<<1, SCAN_THREADS, 0, s>>>(a, v, *finish);
     } else {
-        paths_kernel<<<grid_for(n, 256, num_sms, 8), 256, 0, s>>>(a, v);
+        verb_scan_kernel<<<grid_for(verbs_hint, SCAN_TILE, num_sms, 4), SCAN_THREADS, 0, s>>>(a, v);
+        if (finish) {
+            finish_kernel<false><<<1, SCAN_THREADS, 0, s>>>(a, v, *finish);
+        } else {
+            paths_kernel<<<grid_for(n, 256, num_sms, 8), 256, 0, s>>>(a, v);
+        }
+        note_launches(1);
     }
-    note_launches(1);
+    if (advance) join_stroke_advance(side, s);
     return cudaGetLastError();
 }
 
@@ -1756,7 +1759,10 @@ cudaError_t launch_stroke_verbs_emit(const StrokeArgs& a, const StrokeVerbs& v,
                                      const SideStreams& side, cudaStream_t s) {
     if (a.widths || a.sources) return launch_stroke_steps_emit(a, v, verbs_hint, num_sms, side, s);
     if (a.vertex_attrs) {
-        launch_stroke_advance(a, v, num_sms, side, s);
+        if (a.num_paths > STROKE_ADVANCE_EARLY) {
+            launch_stroke_advance(a, v, num_sms, side, s);
+            join_stroke_advance(side, s);
+        }
         launch_verbs_emit<true>(a, v, verbs_hint, runs, num_sms, side, s);
     } else {
         launch_verbs_emit<false>(a, v, verbs_hint, runs, num_sms, side, s);

@@ -74,3 +74,12 @@ def test_tiles(ctx, n):
     sv.check(ctx, batch, o)
     for how in ("widths", "sources records"):
         sv.same_bits(sv.stepped(ctx, batch, o, how, by_path=True), sv.stepped(ctx, batch, o, how))
+
+
+@pytest.mark.parametrize("how", ["records", "sources records"])
+@pytest.mark.parametrize("n", [12288, 12289])
+def test_sums_beside_the_count_or_after_it(ctx, how, n):
+    batch = rows([[2, 3], [1], [40, 40]] * (n // 3) + [[1]] * (n % 3), n)
+    o = sv.options(np.random.default_rng(n), batch.num_paths, tol=0.1)
+    o["line_width"] = np.maximum(o["line_width"], 0.3)
+    sv.same_bits(sv.stepped(ctx, batch, o, how, by_path=True), sv.stepped(ctx, batch, o, how))
