@@ -5,7 +5,8 @@
 //      ones first. A warp builds its path's event queue, sorts it, runs the sweep and triangulates
 //      the spans (fill_warp.cuh) in its private heap; at the end it reserves room in a staging
 //      pool with one atomic add per array and writes vertices and triangles (path-relative ids)
-//      there. Large batches' tiny paths go to fill_sweep_kernel, a thread each (fill_sweep.cuh).
+//      there. Large batches' small, simple paths go to fill_sweep_kernel, a thread each
+//      (fill_sweep.cuh).
 //   2. the caller's index-range check and look-back scan turn the per-path counts into offsets;
 //   3. fill_emit_kernel: one warp per path copies the staged vertices to their final place and
 //      the indices with the path's id base added (u16 or u32).
@@ -37,40 +38,87 @@ constexpr uint32_t FILL_SWEEPERS_PER_SM = LG_FILL_SWEEPERS_PER_SM;
 // Heaps of all sweepers together stay under this many bytes (fewer blocks when larger).
 constexpr size_t FILL_HEAP_POOL_BYTES = 16ull << 30;
 
-// Paths of lines only with fewer than TINY_POINTS points, when there are TINY_MIN_PATHS of them or
-// more, are swept by a thread each (fill_sweep.cuh), TINY_LANES of a warp's. A warp's sweep of such a
-// path is mostly what every path costs (its arrays, the steps around each event), and that code goes
-// through the instruction cache once per path: a thread per path shares each fetch. Microseconds for
-// a batch by warps and by threads: triangles 20,000 248 and 180, 80,000 730 and 379, 200,000 1708 and
-// 854; quadrilaterals 10,000 186 and 216, 20,000 305 and 258, 200,000 2392 and 1795; hexagons 80,000
-// 1295 and 1207; octagons 80,000 1662 and 1695, 200,000 4106 and 4368. Of 1, 4, 8, 12, 16 and 32
-// threads of a warp 12 were fastest.
-constexpr uint32_t TINY_POINTS = 8;  // a power of two: a bin of the size order
-constexpr uint32_t TINY_MIN_PATHS = 16384;
+// Small, simple paths of large batches are swept by a thread each (fill_sweep.cuh), TINY_LANES of a
+// warp's. A warp's sweep of such a path is mostly what every path costs (its arrays, the steps around
+// each event), and that code goes through the instruction cache once per path: a thread per path shares
+// each fetch. A path with many edges side by side is the warp's: it looks at 32 at once. Small: fewer
+// than TINY_SIZE points and edges of curves, the latter counted TINY_CURVE times, or
+// TINY_CURVE_MANY times from TINY_MANY_PATHS paths on; simple: at most TINY_PEAKS (TINY_PEAKS_MANY)
+// local maxima of the sweep's coordinate; and TINY_MIN_PATHS such paths or more. Microseconds by warps
+// and by threads:
+//   convex polygons of 8 points: 9,000 219 and 262, 12,500 284 and 261, 100,000 1718 and 912; of 62,
+//     12,500 1414 and 1310, 30,000 3112 and 1773; of 100, 30,000 4896 and 2830;
+//   eight points at random distances around a centre: 12,500 298 and 421, 30,000 638 and 549; 16:
+//     1314 and 1695; combs of 12 teeth, 30,000: 1623 and 3227;
+//   outlines of four cubics: 12,500 1044 and 1418, 30,000 2443 and 1429.
+constexpr uint32_t TINY_SIZE = 1u << 7;  // a power of two: a bin of the size order
+constexpr uint32_t TINY_BIN = 32u - 7u;
+constexpr uint32_t TINY_MANY_PATHS = 24576;
+constexpr uint32_t TINY_PEAKS = 2, TINY_PEAKS_MANY = 3;
+constexpr uint32_t TINY_CURVE = 4, TINY_CURVE_MANY = 2;
+constexpr uint32_t TINY_MIN_PATHS = 12288;
 constexpr uint32_t TINY_LANES = 12;
+static_assert(TINY_SIZE == 1u << (32u - TINY_BIN), "bins from there on hold the smaller paths");
 
-// Of the size order's counters: the number of paths with fewer than TINY_POINTS points.
+// Of the size order's counters: the number of tiny paths.
 __device__ __forceinline__ uint32_t tiny_paths(const uint32_t* counters) {
     uint32_t n = 0;
-    for (uint32_t b = 32u - 3u; b < SIZE_ORDER_BINS; ++b) n += counters[b];
+    for (uint32_t b = TINY_BIN; b < SIZE_ORDER_BINS; ++b) n += counters[b];
     return n;
 }
-static_assert(TINY_POINTS == 1u << 3, "bins 29 and up hold paths of fewer than 8 points");
 
-// Sizes for the size order: points, at least TINY_POINTS for a path with a curve.
-__global__ void fill_sizes_kernel(const uint8_t* verbs, const uint32_t* verb_offsets,
-                                  const uint32_t* point_offsets, uint32_t n, uint32_t* sizes) {
+// Sizes for the size order: points, and in the bins before theirs those of the paths that are not tiny.
+__global__ void fill_sizes_kernel(const uint8_t* verbs, const float* points,
+                                  const uint32_t* verb_offsets, const uint32_t* point_offsets,
+                                  uint32_t n, const lyon_fill_options* options,
+                                  uint32_t num_options, uint32_t* sizes) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t size = point_offsets[i + 1] - point_offsets[i];
-    if (size < TINY_POINTS) {
+    const uint32_t p0 = point_offsets[i], p1 = point_offsets[i + 1];
+    const uint32_t large = max(min(p1 - p0, ~0u / (2u * TINY_SIZE)), 1u) * (2u * TINY_SIZE);
+    uint32_t size = p1 - p0;
+    if (size < TINY_SIZE) {
+        const lyon_fill_options o = options[num_options > 1 ? i : 0];
+        const uint32_t along = o.sweep_orientation == LYON_ORIENTATION_HORIZONTAL ? 0u : 1u;
+        const bool many = n >= TINY_MANY_PATHS;
+        const uint32_t weight = many ? TINY_CURVE_MANY : TINY_CURVE;
         const uint32_t v0 = verb_offsets[i], v1 = verb_offsets[i + 1];
-        bool tiny = v1 - v0 <= 2 * TINY_POINTS;
-        for (uint32_t v = v0; tiny && v < v1; ++v)
-            tiny = verbs[v] != LYON_VERB_QUADRATIC_TO && verbs[v] != LYON_VERB_CUBIC_TO;
-        if (!tiny) size = TINY_POINTS;
+        if (v1 - v0 > 2 * TINY_SIZE) size = TINY_SIZE;
+        uint32_t p = p0, peaks = 0;
+        float before = 0.0f;
+        bool rising = false;
+        V2 q[4];
+        q[3] = V2{0.0f, 0.0f};
+        for (uint32_t v = v0; size < TINY_SIZE && v < v1; ++v) {
+            const uint32_t k = verbs[v];
+            const uint32_t np = k == LYON_VERB_QUADRATIC_TO ? 2u : k == LYON_VERB_CUBIC_TO ? 3u
+                                : k == LYON_VERB_END ? 0u : 1u;
+            if (p + np > p1) break;
+            q[0] = q[3];
+            for (uint32_t j = 0; j < np; ++j) {
+                const size_t at = 2 * ((size_t)p + j);
+                const V2 x = V2{points[at], points[at + 1]};
+                q[j + 1] = x;
+                const float c = along ? x.y : x.x;
+                if (k == LYON_VERB_BEGIN || c > before) {
+                    rising = true;
+                } else if (c < before && rising) {
+                    rising = false;
+                    ++peaks;
+                }
+                before = c;
+            }
+            if (np > 1u) {
+                const float m = np == 2u ? quad_wang(q[0], q[1], q[2], o.tolerance)
+                                         : cubic_wang(q[0], q[1], q[2], q[3], o.tolerance);
+                size += weight * min(to_u32_or1(m), TINY_SIZE);
+            }
+            if (np > 0u) q[3] = q[np];
+            if (peaks > (many ? TINY_PEAKS_MANY : TINY_PEAKS)) size = TINY_SIZE;
+            p += np;
+        }
     }
-    sizes[i] = size;
+    sizes[i] = size < TINY_SIZE ? size : large;
 }
 
 struct SweepArgs {
@@ -403,7 +451,8 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
     const bool tiny = n >= fillk::TINY_MIN_PATHS;
     if (tiny) {  // (the sizes lie in the first retry list, which is written after the order)
         fillk::fill_sizes_kernel<<<(n + 255) / 256, 256, 0, stream>>>(
-            batch->verbs, batch->verb_offsets, batch->point_offsets, n, lists[0]);
+            batch->verbs, batch->points, batch->verb_offsets, batch->point_offsets, n, options,
+            num_options, lists[0]);
         lg::note_launches(1);
     }
     if (launch_size_order(batch->point_offsets, n, size_cls, lists[1], size_counters, stream,
