@@ -686,8 +686,8 @@ int lyon_gpu_coverage_compare(const float* boxes, uint32_t num_paths, uint32_t g
 
 /* ---- Stroke launch settings and autotuner (no lyon counterpart) ---------------------------- */
 
-/* Runtime settings of the stroke kernels that take a path as a whole, which are for the paths that the
- * verb-parallel stroke leaves. */
+/* Runtime settings of the stroke kernels that take a path as a whole: for batches of many short paths,
+ * and for the paths that the verb-parallel stroke leaves. */
 typedef struct lyon_gpu_stroke_tuning {
     uint32_t long_path_points;  /* paths with more points are scheduled first (so that no long
                                    path is left running alone at the end of a launch);
@@ -702,8 +702,8 @@ typedef struct lyon_gpu_stroke_tuning {
 int lyon_gpu_set_stroke_tuning(lyon_gpu_context* ctx, const lyon_gpu_stroke_tuning* tuning);
 int lyon_gpu_get_stroke_tuning(lyon_gpu_context* ctx, lyon_gpu_stroke_tuning* tuning);
 
-/* Times the batched stroke (device buffers, u32 per-path indices) on the first `sample_paths`
- * paths of `batch` (0: all) for each candidate setting — long_path_points in {0, 256, 1024,
+/* Times the batched stroke, path by path (device buffers, u32 per-path indices), on the first
+ * `sample_paths` paths of `batch` (0: all) for each candidate setting — long_path_points in {0, 256, 1024,
  * 8192} x blocks_per_sm in {as many as fit, 1} x short_path_points in {0, 32} — and keeps the
  * fastest on the context, so that later calls on paths of the same length distribution use it.
  * `best` receives the choice; `times_ms` (optional, 16 entries) the candidates' times in that

@@ -70,7 +70,8 @@ struct lyon_gpu_context {
     bool verbs_valid = false;   // the last count phase was verb-parallel
     bool verb_runs = false;     // its batch has curves with interior steps
     uint32_t walk_paths = 0;    // its paths left to the walk
-    // stroke launch settings (the autotuner's knobs)
+    // stroke launch settings (the autotuner's knobs), of the path-by-path stroke
+    bool force_by_path = false;        // no batch goes verb by verb (the autotuner, for its times)
     uint32_t long_path_points = 1024;  // paths with more points go first; 0: path order
     uint32_t blocks_per_sm = 0;        // 0: as many as fit
     uint32_t short_path_points = 32;   // line-only paths up to this size: one per thread
@@ -617,7 +618,7 @@ int pipeline_count(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch
     ctx->split_valid = false;
     ctx->verbs_valid = false;
     uint32_t verbs = ctx->verbs_known;
-    bool by_path = kind != KIND_STROKE || n == 0;
+    bool by_path = kind != KIND_STROKE || n == 0 || ctx->force_by_path;
     if (!by_path && may_be_sooner(ctx, n)) {
         lg::BatchShape shape;
         if (!batch_shape(ctx, batch, &shape)) return LYON_ERR_CUDA;
@@ -1325,6 +1326,7 @@ int lyon_gpu_autotune_stroke(lyon_gpu_context* ctx, const lyon_path_batch* batch
     lyon_gpu_get_stroke_tuning(ctx, &saved);
     const bool saved_timing = ctx->timing;
     ctx->timing = false;
+    ctx->force_by_path = true;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1360,6 +1362,7 @@ int lyon_gpu_autotune_stroke(lyon_gpu_context* ctx, const lyon_path_batch* batch
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ctx->timing = saved_timing;
+    ctx->force_by_path = false;
     if (rc != LYON_OK) {
         lyon_gpu_set_stroke_tuning(ctx, &saved);
         return rc;
