@@ -715,12 +715,12 @@ int lyon_gpu_autotune_stroke(lyon_gpu_context* ctx, const lyon_path_batch* batch
                              float* times_ms, uint32_t* num_candidates);
 
 /* Runtime settings of the fill sweep on a context: lyon's sweep of one path runs on one warp (a
- * block). In batches of 16,384 or more paths of lines with fewer than 8 points those paths are swept
- * by one thread each, several of a block. */
+ * block). In batches of 12,288 or more small, simple paths those are swept by one thread each, several
+ * of a block. */
 typedef struct lyon_gpu_fill_tuning {
     uint32_t blocks_per_sm; /* sweep blocks per SM; 0: the default (16) */
-    uint32_t lanes;         /* threads of a block that sweep tiny paths: 1 to 32; 0: chosen per launch
-                               from its paths per block, up to 12 */
+    uint32_t lanes;         /* threads of a block that sweep small paths: 1 to 32; 0: chosen per
+                               launch from its paths per block, up to 12 */
 } lyon_gpu_fill_tuning;
 
 int lyon_gpu_set_fill_tuning(lyon_gpu_context* ctx, const lyon_gpu_fill_tuning* tuning);
@@ -730,8 +730,9 @@ int lyon_gpu_get_fill_tuning(lyon_gpu_context* ctx, lyon_gpu_fill_tuning* tuning
  * paths of `batch` (0: all) for each candidate setting — blocks_per_sm in {16, 8} x lanes in
  * {1, 4, 8, 12, 16} — and keeps the fastest on the context, so that later calls on paths of the
  * same size distribution use it. `best` receives the choice, `times_ms` (optional, 10 entries, lanes
- * varying fastest) the candidates' times, `num_candidates` the count. Outputs do not depend on the
- * settings. */
+ * varying fastest) the candidates' times, `num_candidates` the count. On a sample without paths that
+ * threads sweep, `lanes` stays chosen per launch (`best` gives the most it takes, 12). Outputs do not
+ * depend on the settings. */
 int lyon_gpu_autotune_fill(lyon_gpu_context* ctx, const lyon_path_batch* batch,
                            const lyon_fill_options* options, uint32_t num_options,
                            uint32_t sample_paths, lyon_gpu_fill_tuning* best, float* times_ms,

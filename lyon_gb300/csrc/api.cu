@@ -1436,7 +1436,13 @@ int lyon_gpu_autotune_fill(lyon_gpu_context* ctx, const lyon_path_batch* batch,
         lyon_gpu_set_fill_tuning(ctx, &saved);
         return rc;
     }
-    lyon_gpu_set_fill_tuning(ctx, &b);
+    // A sample without paths that threads sweep says nothing about their number.
+    lyon_gpu_fill_tuning keep = b;
+    if (!ctx->fill.by_threads) {
+        keep.lanes = 0;
+        b.lanes = lg::FILL_LANES;
+    }
+    lyon_gpu_set_fill_tuning(ctx, &keep);
     if (best) *best = b;
     return LYON_OK;
 }

@@ -38,7 +38,7 @@ constexpr uint32_t FILL_SWEEPERS_PER_SM = LG_FILL_SWEEPERS_PER_SM;
 // Heaps of all sweepers together stay under this many bytes (fewer blocks when larger).
 constexpr size_t FILL_HEAP_POOL_BYTES = 16ull << 30;
 
-// Small, simple paths of large batches are swept by a thread each (fill_sweep.cuh), TINY_LANES of a
+// Small, simple paths of large batches are swept by a thread each (fill_sweep.cuh), FILL_LANES of a
 // warp's. A warp's sweep of such a path is mostly what every path costs (its arrays, the steps around
 // each event), and that code goes through the instruction cache once per path: a thread per path shares
 // each fetch. A path with many edges side by side is the warp's: it looks at 32 at once. Small: fewer
@@ -57,7 +57,6 @@ constexpr uint32_t TINY_MANY_PATHS = 24576;
 constexpr uint32_t TINY_PEAKS = 2, TINY_PEAKS_MANY = 3;
 constexpr uint32_t TINY_CURVE = 4, TINY_CURVE_MANY = 2;
 constexpr uint32_t TINY_MIN_PATHS = 12288;
-constexpr uint32_t TINY_LANES = 12;
 static_assert(TINY_SIZE == 1u << (32u - TINY_BIN), "bins from there on hold the smaller paths");
 
 // Of the size order's counters: the number of tiny paths.
@@ -460,8 +459,8 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
         order = lists[1];
     uint32_t items = n;
     // Threads of a block that sweep tiny paths: as many as the launch has paths per block, up to
-    // TINY_LANES (LYON_GB300_FILL_LANES or the context's setting force a number, 1 to 32).
-    uint32_t lanes = std::max<uint32_t>(1u, std::min<uint32_t>(fillk::TINY_LANES, n / threads));
+    // FILL_LANES (LYON_GB300_FILL_LANES or the context's setting force a number, 1 to 32).
+    uint32_t lanes = std::max<uint32_t>(1u, std::min<uint32_t>(FILL_LANES, n / threads));
     if (fb.lanes >= 1 && fb.lanes <= 32) lanes = fb.lanes;
     if (const char* env = getenv("LYON_GB300_FILL_LANES")) {
         const long v = strtol(env, nullptr, 10);
@@ -541,6 +540,7 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
             if (error) *error = std::string("fill sweep: ") + cudaGetErrorString(e);
             return LYON_ERR_CUDA;
         }
+        if (attempt == 0) fb.by_threads = h.ctl[3] > 0;
         if (h.ctl[1] == 0) break;
         // Some paths ran out of heap or staging room: more of both, then only those paths.
         // The staging tops stay where they are (the failed reservations are abandoned).

@@ -9,6 +9,9 @@
 
 namespace lg {
 
+// Most threads of a block that sweep small paths, when the caller sets no number.
+constexpr uint32_t FILL_LANES = 12;
+
 // Device buffers the fill pipeline keeps between its count and emit phases.
 struct FillBuffers {
     void* scratch = nullptr;        // sweep heaps, one per warp
@@ -29,6 +32,7 @@ struct FillBuffers {
     // Threads of a one-warp block that sweep tiny paths (1..32); 0: chosen per launch from its paths
     // per block.
     uint32_t lanes = 0;
+    bool by_threads = false;        // the last batch had paths that threads swept
     // When set, every buffer here comes from this pool in stream order (serving contexts).
     cudaMemPool_t pool = nullptr;
     // Vertex sources (FillVertex::sources), when a call asks for them:

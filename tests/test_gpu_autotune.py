@@ -52,3 +52,24 @@ def test_stroke_settings_are_timed_path_by_path(ctx):
     T.tessellate_paths("stroke", db, od, len(opts), 32, T.INDEX_GLOBAL, 0, ctx)
     ctx.lib.lyon_gpu_last_timings(ctx.h, ms)
     assert ms[3] < min(times) / 2
+
+
+@pytest.mark.parametrize("threads", [False, True])
+def test_fill_keeps_the_number_of_threads_only_where_it_matters(ctx, threads):
+    if threads:
+        batch, opts = routes.lines(20000, 4, 2, closed=True), None
+    else:
+        batch, opts = workloads.glyph_fill(300, seed=47)
+    if opts is None:
+        opts = workloads.glyph_fill(1, seed=1)[1][:1]
+    db, od = T.DeviceBatch.upload(batch, 0), T.upload_options(opts, 0)
+    best, now, nc = _native.CFillTuning(), _native.CFillTuning(), ctypes.c_uint32()
+    times = (ctypes.c_float * 10)()
+    cb = db.c()
+    r = ctx.lib.lyon_gpu_autotune_fill(ctx.h, ctypes.byref(cb), od.data_ptr(), len(opts), 0,
+                                       ctypes.byref(best), times, ctypes.byref(nc))
+    assert r == T.LYON_OK and nc.value == 10 and min(times) > 0
+    assert ctx.lib.lyon_gpu_get_fill_tuning(ctx.h, ctypes.byref(now)) == 0
+    assert now.blocks_per_sm == best.blocks_per_sm
+    assert best.lanes in (1, 4, 8, 12, 16)
+    assert now.lanes == (best.lanes if threads else 0)
