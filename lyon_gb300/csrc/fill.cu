@@ -468,7 +468,11 @@ int fill_count(FillBuffers& fb, const lyon_path_batch* batch, const lyon_fill_op
     }
     const int MAX_ATTEMPTS = 4;
     for (int attempt = 0; attempt < MAX_ATTEMPTS; ++attempt) {
-        uint32_t nthreads = threads;
+        // No more heaps than there are paths (in powers of two, so that batches that grow little by
+        // little do not each allocate them anew).
+        uint32_t nthreads = 1;
+        while (nthreads < items && nthreads < threads) nthreads *= 2;
+        nthreads = std::min(nthreads, threads);
         size_t heap_bytes = (size_t)fb.heap_words * 4 * nthreads;
         // Keep the heaps under the pool size: fewer blocks when each heap is large.
         while (heap_bytes > fillk::FILL_HEAP_POOL_BYTES && nthreads > 4) {
