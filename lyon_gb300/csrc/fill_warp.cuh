@@ -1283,7 +1283,7 @@ struct WarpFiller {
             }
             uint2 s = make_uint2(0u, 0u);
             if (live) s = spans[idx];
-            __syncwarp();  // two lanes may have the same span, and one of them writes it
+            if (ve_n > 1 && ve_span0 == ve_span1) __syncwarp();  // lane 1 writes what lane 0 reads
             if (live) {
                 const uint32_t again = (ve_n > 0 && i > 0 && idx == ve_span0 ? 1u : 0u) +
                                        (ve_n > 1 && i > 1 && idx == ve_span1 ? 1u : 0u);
