@@ -1267,6 +1267,7 @@ struct WarpFiller {
     __device__ __forceinline__ void process_edges_above() {
         // The vertex joins the lists of the vertex events' spans, then ends those to end: a lane
         // each. A span that is met twice takes it twice.
+        const bool twice = ve_n > 1 && ve_span0 == ve_span1;
 #pragma unroll 1
         for (uint32_t base = 0; base < ve_n + end_n; base += 32) {
             const uint32_t i = base + lane;
@@ -1281,10 +1282,8 @@ struct WarpFiller {
                 fail(FILL_ERR_HEAP);
                 return;
             }
-            uint2 s = make_uint2(0u, 0u);
-            if (live) s = spans[idx];
-            if (ve_n > 1 && ve_span0 == ve_span1) __syncwarp();  // lane 1 writes what lane 0 reads
             if (live) {
+                const uint2 s = spans[idx];
                 const uint32_t again = (ve_n > 0 && i > 0 && idx == ve_span0 ? 1u : 0u) +
                                        (ve_n > 1 && i > 1 && idx == ve_span1 ? 1u : 0u);
                 const int side = i == 0 && !end ? ve_side0 : LEFT;
@@ -1293,11 +1292,16 @@ struct WarpFiller {
                 if (end) {
                     S.span_len[s.x].x = s.y + again + 1u;
                     S.flushed[flushed_n + i - ve_n] = s.x;
-                } else if (!ends && !(i == 0 && ve_n > 1 && ve_span1 == idx)) {
-                    spans[idx].y = s.y + again + 1u;
+                } else if (!ends && !twice) {
+                    spans[idx].y = s.y + 1u;
                 }
             }
             node_n += ve_n + end_n - base < 32u ? ve_n + end_n - base : 32u;
+            __syncwarp();
+        }
+        // (Both lanes have read the span: one of them cannot write it before.)
+        if (twice && (ve_span0 < end_first || ve_span0 - end_first >= (int32_t)end_n)) {
+            if (lane == 0) spans[ve_span0].y += 2u;
             __syncwarp();
         }
         flushed_n += end_n;
