@@ -467,6 +467,23 @@ bool grow_verbs(lyon_gpu_context* ctx, uint32_t verbs) {
     return true;
 }
 
+// Gives the verbs' arrays back; false when there are none.
+bool give_back_verbs(lyon_gpu_context* ctx) {
+    DevBuf& b = ctx->verb_mem;
+    if (!b.ptr) return false;
+    if (b.pooled) {
+        cudaFreeAsync(b.ptr, ctx->stream);
+    } else {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(b.ptr);
+    }
+    b.ptr = nullptr;
+    b.cap = 0;
+    ctx->verb_cap = 0;
+    ctx->verbs_valid = false;
+    return true;
+}
+
 const lg::SideStreams& side_streams(lyon_gpu_context* ctx) {
     if (!ctx->side_made) {
         ctx->side_made = true;
@@ -810,12 +827,24 @@ int batched_device(lyon_gpu_context* ctx, int kind, const lyon_path_batch* batch
         r = fill_source_offsets(ctx, batch->num_paths, tv);
         if (r != LYON_OK) return r;
     }
-    const uint64_t nsrc = kind == KIND_FILL ? ctx->total_sources : tv;
-    if (!ensure(ctx, ctx->out_vertices, tv * vbytes + 16) ||
-        !ensure(ctx, ctx->out_indices, ti * (index_bits / 8) + 16) ||
-        (ctx->want_sources &&
-         !ensure(ctx, ctx->out_sources, nsrc * sizeof(lyon_vertex_source) + 16)))
-        return LYON_ERR_OUT_OF_MEMORY;
+    auto room = [&]() {
+        const uint64_t nsrc = kind == KIND_FILL ? ctx->total_sources : tv;
+        return ensure(ctx, ctx->out_vertices, tv * vbytes + 16) &&
+               ensure(ctx, ctx->out_indices, ti * (index_bits / 8) + 16) &&
+               (!ctx->want_sources ||
+                ensure(ctx, ctx->out_sources, nsrc * sizeof(lyon_vertex_source) + 16));
+    };
+    if (!room()) {
+        // The verbs' arrays may be what is in the way: path by path the stroke needs none.
+        if (!give_back_verbs(ctx) || kind != KIND_STROKE) return LYON_ERR_OUT_OF_MEMORY;
+        const bool forced = ctx->force_by_path;
+        ctx->force_by_path = true;
+        r = pipeline_count(ctx, kind, batch, options, num_options, index_bits, index_mode,
+                           vertex_offset, &tv, &ti, &failed);
+        ctx->force_by_path = forced;
+        if (r != LYON_OK) return r;
+        if (!room()) return LYON_ERR_OUT_OF_MEMORY;
+    }
     r = pipeline_emit(ctx, kind, batch, options, num_options, index_bits, index_mode,
                       vertex_offset, as<float>(ctx->out_vertices), ctx->out_indices.ptr, tv);
     if (r != LYON_OK) return r;
