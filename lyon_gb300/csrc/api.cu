@@ -569,6 +569,7 @@ bool batch_shape(lyon_gpu_context* ctx, const lyon_path_batch* batch, lg::BatchS
 // false when the batch is left to the path-by-path count (its offsets overlap, or no room for the
 // arrays).
 // `need`: the batch's verbs, 0 when they are not known.
+constexpr uint32_t FEW_PATHS = 32;
 int count_by_verb(lyon_gpu_context* ctx, const lyon_path_batch* batch,
                   const lyon_stroke_options* options, uint32_t num_options, int index_bits,
                   int index_mode, uint64_t vertex_offset, uint32_t need, uint64_t* tv,
@@ -590,7 +591,13 @@ int count_by_verb(lyon_gpu_context* ctx, const lyon_path_batch* batch,
         const lg::StrokeVerbs v = stroke_verbs(ctx, n);
         const lg::StrokeArgs a = stroke_args(ctx, batch, options, num_options, index_bits,
                                              index_mode, vertex_offset);
-        const uint32_t hint = need ? need : ctx->verb_count > n ? ctx->verb_count : n;
+        // Grids for the verbs of this batch, and where the caller does not say how many they are, for
+        // as many as there is room for: sized by the last batch instead, 2,000 polylines of 500
+        // points after a single line took 3293 us instead of 276 (and path by path 402). A few paths
+        // may be taken for a small batch: their walk path by path would be longer all the same, and
+        // the full grids cost a small batch 6 us.
+        const uint32_t last = ctx->verb_count > n ? ctx->verb_count : n;
+        const uint32_t hint = need ? need : n <= FEW_PATHS && last < v.cap ? last : v.cap;
         lg::StrokeFinish f{};
         const lg::StrokeFinish* finish = nullptr;
         if (n <= lg::STROKE_FINISH_PATHS && ensure_host(ctx, ctx->h_small, 64)) {

@@ -126,3 +126,59 @@ def test_time_of_many_short_lines(ctx, how):
     t, path = best(batch), best(PathBatch(batch.verbs, batch.points, vo, po))
     print(how, t, path)
     assert t < 1.25 * path
+
+
+def test_a_large_batch_after_a_small_one(ctx):
+    # A context that has room for the large batch does not know its size beforehand.
+    large, small = lines(2000, 500, 4), lines(1, 2, 5)
+    od = T.upload_options(opts_for(large)[:1], 0)
+    dl, ds = T.DeviceBatch.upload(large, 0), T.DeviceBatch.upload(small, 0)
+
+    def call(db):
+        t = time.perf_counter()
+        res = T.tessellate_paths("stroke", db, od, 1, 32, T.INDEX_GLOBAL, 0, ctx)
+        ctx.synchronize()
+        return time.perf_counter() - t, res
+    call(dl)
+    again = min(call(dl)[0] for _ in range(5))
+    want = call(dl)[1].vertices().clone()
+    after = []
+    for _ in range(5):
+        call(ds)
+        t, res = call(dl)
+        after.append(t)
+    assert bool((res.vertices() == want).all())
+    print(again, after)
+    assert min(after) < 2 * again
+
+
+@pytest.mark.parametrize("how", ["positions", "records"])
+def test_settings_of_the_path_by_path_stroke(ctx, how):
+    # Short line-only paths by a thread each, long ones first, one block per SM: the same outputs,
+    # and those of the walk by one warp. (A last path whose offsets run backwards sends all of them
+    # path by path.)
+    import ctypes
+    from lyon_gb300 import _native
+    batch = sv.rough_paths(800, 9)
+    short = lines(700, 5, 3)
+    verbs = np.concatenate([batch.verbs, short.verbs])
+    pts = np.concatenate([batch.points, short.points])
+    vo = np.concatenate([batch.verb_offsets, short.verb_offsets[1:] + batch.verb_offsets[-1]])
+    po = np.concatenate([batch.point_offsets, short.point_offsets[1:] + batch.point_offsets[-1]])
+    vo, po = np.append(vo, vo[-1] - 1), np.append(po, po[-1])
+    b = PathBatch(verbs, pts, vo.astype(np.uint32), po.astype(np.uint32))
+    o = opts_for(b)
+    saved = _native.CStrokeTuning()
+    ctx.lib.lyon_gpu_get_stroke_tuning(ctx.h, ctypes.byref(saved))
+    out = []
+    try:
+        for tuning in ((0, 0, 0), (1024, 0, 32), (16, 1, 64), (0, 2, 5)):
+            t = _native.CStrokeTuning(*tuning)
+            assert ctx.lib.lyon_gpu_set_stroke_tuning(ctx.h, ctypes.byref(t)) == T.LYON_OK
+            if how == "positions":
+                sv.check(ctx, b, o)
+            out.append(sv.stepped(ctx, b, o, "records" if how == "records" else "widths"))
+    finally:
+        ctx.lib.lyon_gpu_set_stroke_tuning(ctx.h, ctypes.byref(saved))
+    for x in out[1:]:
+        sv.same_bits(out[0], x)
