@@ -44,8 +44,10 @@ constexpr size_t FILL_HEAP_POOL_BYTES = 16ull << 30;
 // each fetch. A path with many edges side by side is the warp's: it looks at 32 at once. Small: fewer
 // than TINY_SIZE points and edges of curves, the latter counted TINY_CURVE times, or
 // TINY_CURVE_MANY times from TINY_MANY_PATHS paths on; simple: at most TINY_PEAKS (TINY_PEAKS_MANY)
-// local maxima of the sweep's coordinate; and TINY_MIN_PATHS such paths or more. Microseconds by warps
-// and by threads:
+// local maxima of the sweep's coordinate; and TINY_MIN_PATHS such paths or more, at least half of the
+// batch (their sweep follows that of the others, and the longest of them takes milliseconds by one
+// thread: 50,000 glyphs, a quarter of them small and simple, 82 and 90 ms). Microseconds by warps and by
+// threads:
 //   convex polygons of 8 points: 9,000 219 and 262, 12,500 284 and 261, 100,000 1718 and 912; of 62,
 //     12,500 1414 and 1310, 30,000 3112 and 1773; of 100, 30,000 4896 and 2830;
 //   eight points at random distances around a centre: 12,500 298 and 421, 30,000 638 and 549; 16:
@@ -59,11 +61,12 @@ constexpr uint32_t TINY_CURVE = 4, TINY_CURVE_MANY = 2;
 constexpr uint32_t TINY_MIN_PATHS = 12288;
 static_assert(TINY_SIZE == 1u << (32u - TINY_BIN), "bins from there on hold the smaller paths");
 
-// Of the size order's counters: the number of tiny paths.
-__device__ __forceinline__ uint32_t tiny_paths(const uint32_t* counters) {
-    uint32_t n = 0;
-    for (uint32_t b = TINY_BIN; b < SIZE_ORDER_BINS; ++b) n += counters[b];
-    return n;
+// Of the size order's counters: how many of the n paths are swept by threads.
+__device__ __forceinline__ uint32_t tiny_paths(const uint32_t* counters, uint32_t n) {
+    if (!counters) return 0;
+    uint32_t tiny = 0;
+    for (uint32_t b = TINY_BIN; b < SIZE_ORDER_BINS; ++b) tiny += counters[b];
+    return tiny >= TINY_MIN_PATHS && tiny >= n / 2u ? tiny : 0u;
 }
 
 // Sizes for the size order: points, and in the bins before theirs those of the paths that are not tiny.
@@ -161,8 +164,7 @@ __global__ void __launch_bounds__(32, LG_FILL_MIN_BLOCKS) fill_warp_kernel(Sweep
     const uint32_t lane = threadIdx.x;
     WarpFiller<SRC> f(smem);
     uint32_t* heap = A.heaps + (size_t)blockIdx.x * A.heap_words;
-    const uint32_t tiny = A.size_counters ? tiny_paths(A.size_counters) : 0u;
-    const uint32_t num_items = A.num_items - (tiny >= TINY_MIN_PATHS ? tiny : 0u);
+    const uint32_t num_items = A.num_items - tiny_paths(A.size_counters, A.num_items);
     for (;;) {
         uint32_t item = 0;
         if (lane == 0) item = atomicAdd(&A.counters[0], 1u);
@@ -236,8 +238,8 @@ __global__ void __launch_bounds__(32, LG_FILL_MIN_BLOCKS) fill_sweep_kernel(Swee
     // Each of the block's first `lanes` threads sweeps its own paths with its own heap. The
     // sweep's control flow depends on the path, so lanes diverge; where they run the same code
     // (the event loop's common steps) one instruction fetch serves several paths.
-    const uint32_t tiny = A.size_counters ? tiny_paths(A.size_counters) : 0u;
-    if (threadIdx.x >= A.lanes || tiny < TINY_MIN_PATHS) return;
+    const uint32_t tiny = tiny_paths(A.size_counters, A.num_items);
+    if (threadIdx.x >= A.lanes || tiny == 0) return;
     const uint32_t first = A.num_items - tiny;
     const uint32_t wid = blockIdx.x * A.lanes + threadIdx.x;
     FillerT<SRC> f;

@@ -83,6 +83,25 @@ def test_small_paths(simple, orientation):
     assert np.array_equal(s["gpu"]["vertices"], s["oracle"]["vertices"], equal_nan=True)
 
 
+@pytest.mark.parametrize("others", [13000, 13600])
+def test_small_paths_among_as_many_others(others):
+    # Threads sweep them while they are half of the batch.
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import gpu_helpers
+    rng = np.random.default_rng(others)
+    kinds, comb = [_simple(i, rng) for i in range(256)], _peaks(5, rng)
+    paths = [kinds[i % 256] for i in range(13300)] + [comb] * others
+    paths = [paths[i] for i in rng.permutation(len(paths))]
+    batch = PathBatch.from_paths(paths)
+    opts = fill_options_array([(0.05, FillRule.EvenOdd, 0, 1)])
+    s = gpu_helpers.compare_per_path("fill", batch, opts, index_bits=32, rtol=0.0,
+                                     allow_near_ties=False)
+    assert not s["mismatches"], s["mismatches"][:10]
+    assert np.array_equal(s["gpu"]["vertices"], s["oracle"]["vertices"])
+
+
 def test_time_of_many_simple_paths():
     # 30,000 polygons of 32 points: a thread each takes less time than a warp each would, which is
     # what the same batch takes in three calls of 10,000.
