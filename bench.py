@@ -468,8 +468,8 @@ def run_fill(ctx, args, T, world, batch=None):
         opts = np.zeros(1, dtype=FILL_OPTIONS_DTYPE)
         opts[0] = (0.1, rule, 0, 1)
         od = T.upload_options(opts, 0)
-        # The fill autotuner picks blocks per SM (and the threads of a warp for tiny paths, of which
-        # this batch has none) on a sample of half the batch.
+        # The fill autotuner picks blocks per SM (and the threads of a warp for small simple paths,
+        # if the sample has enough of them) on a sample of half the batch.
         tune = None
         if not args.profile_fill:
             best = _native.CFillTuning()
@@ -546,7 +546,7 @@ def run_fill(ctx, args, T, world, batch=None):
 def run_variable_width(ctx, args, T):
     """Variable line width (StrokeOptions::variable_line_width): the batched-stroke generator's
     paths (seed 2, round joins and caps, tolerance 0.05) with a width factor per point drawn from
-    U[0.5, 2]; one thread per path. CPU baseline: the oracle on a sample."""
+    U[0.5, 2]. CPU baseline: the oracle on a sample."""
     import torch
     from lyon_gb300 import workloads
     from oracle import lyon_oracle as orc
@@ -802,8 +802,8 @@ def run_hatching(ctx, args, T, baseline=True):
 
 def run_polylines(ctx, args, T):
     """Map-like strokes (2,000,000 open polylines, Pareto lengths up to 20,000 points, mixed
-    joins, widths 1-8) at tolerances 0.01, 0.1 and 1.0; for each, the autotuner picks the stroke
-    launch settings on a 200,000-path sample, then the whole batch is timed with them."""
+    joins, widths 1-8) at tolerances 0.01, 0.1 and 1.0; for each, the autotuner picks the launch
+    settings of paths stroked as a whole on a 200,000-path sample, then the whole batch is timed."""
     import torch
     from lyon_gb300 import _native, workloads
     from oracle import lyon_oracle as orc

@@ -593,8 +593,8 @@ typedef struct lyon_srv_config {
                                       caller that waits for requests in submission order while
                                       holding later results can wait forever) */
     uint32_t num_stroke_workers;   /* workers reserved for stroke requests, on streams of the
-                                      device's highest priority and with one stroke block per SM,
-                                      so that their launches start beside running fill sweeps
+                                      device's highest priority (the persistent grid of paths
+                                      stroked as a whole: one block per SM), so that their launches start beside running fill sweeps
                                       instead of queueing behind them; 0 -> none (every worker
                                       takes both kinds, oldest request first) */
     uint32_t fill_blocks_per_sm;   /* fill sweep blocks per SM for each fill worker; 0 -> 8
@@ -715,8 +715,8 @@ int lyon_gpu_autotune_stroke(lyon_gpu_context* ctx, const lyon_path_batch* batch
                              float* times_ms, uint32_t* num_candidates);
 
 /* Runtime settings of the fill sweep on a context: lyon's sweep of one path runs on one warp (a
- * block). In batches of 12,288 or more small, simple paths those are swept by one thread each, several
- * of a block. */
+ * block). In batches that are mostly small, simple paths, 12,288 or more of them, those are swept by one
+ * thread each, several of a block. */
 typedef struct lyon_gpu_fill_tuning {
     uint32_t blocks_per_sm; /* sweep blocks per SM; 0: the default (16) */
     uint32_t lanes;         /* threads of a block that sweep small paths: 1 to 32; 0: chosen per

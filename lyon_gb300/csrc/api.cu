@@ -66,7 +66,7 @@ struct lyon_gpu_context {
     uint32_t verb_cap = 0;      // verbs verb_mem holds
     uint32_t verb_count = 0;    // verbs of the last counted batch
     uint32_t verbs_known = 0;   // the coming batch's verbs when the caller knows them, else 0
-    uint32_t points_known = 0;  // and the points of a batch of one path, when verbs_known is set
+    uint32_t points_known = 0;  // and the points, where the batch is one path from host arrays
     bool verbs_valid = false;   // the last count phase was verb-parallel
     bool verb_runs = false;     // its batch has curves with interior steps
     uint32_t walk_paths = 0;    // its paths left to the walk
@@ -544,7 +544,7 @@ bool may_be_sooner(const lyon_gpu_context* ctx, uint32_t n) {
 
 // The shape of a batch of the device's (one wait for the stream).
 bool batch_shape(lyon_gpu_context* ctx, const lyon_path_batch* batch, lg::BatchShape* out) {
-    if (batch->num_paths == 1 && ctx->verbs_known) {
+    if (batch->num_paths == 1 && ctx->verbs_known && ctx->points_known) {
         *out = lg::BatchShape{ctx->verbs_known, ctx->points_known, ctx->verbs_known,
                               ctx->points_known};
         return true;
@@ -1060,7 +1060,7 @@ int single_path(lyon_gpu_context* ctx, int kind, const uint8_t* verbs, uint32_t 
     ctx->points_known = num_points;
     int r = batched_device(ctx, kind, &b, ctx->in_options.ptr, 1, index_bits,
                            LYON_INDEX_PER_PATH, index_base, &bo);
-    ctx->verbs_known = 0;
+    ctx->verbs_known = ctx->points_known = 0;
     if (r != LYON_OK) return r;
     cudaStream_t s = ctx->stream;
     if (!ensure_host(ctx, ctx->h_small, 64)) return LYON_ERR_OUT_OF_MEMORY;
@@ -1151,8 +1151,9 @@ const int32_t* srv_status(lyon_gpu_context* ctx) { return as<int32_t>(ctx->statu
 cudaStream_t srv_stream(lyon_gpu_context* ctx) { return ctx->stream; }
 
 // Settings of a serving worker's context. A stroke lane gets a stream of the device's highest
-// priority (its blocks are dispatched before queued blocks of other streams) and one stroke block
-// per SM; `fill_blocks_per_sm` (0: default) bounds the fill sweep's residency.
+// priority (its blocks are dispatched before queued blocks of other streams) and one block per SM
+// of the persistent grid for paths stroked as a whole; `fill_blocks_per_sm` (0: default) bounds the
+// fill sweep's residency.
 int srv_configure(lyon_gpu_context* ctx, bool stroke_lane, uint32_t fill_blocks_per_sm,
                   cudaMemPool_t pool) {
     ctx->fill.blocks_per_sm_cap = fill_blocks_per_sm;

@@ -1,4 +1,4 @@
-// fill_sweep.cuh — the fill tessellator's sweep of one path by one thread: the tiny paths of large
+// fill_sweep.cuh — the fill tessellator's sweep of one path by one thread: the small, simple paths of large
 // batches (fill.cu has the rule, fill_warp.cuh the sweep of all others). The Filler runs one path
 // from event-queue construction to the last span flush.
 #pragma once

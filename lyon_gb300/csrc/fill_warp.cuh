@@ -22,7 +22,8 @@
 // warps on an SM, each at another place of 250 KB of code, a warp waited for its next instruction
 // 60 % of the time, so rare steps are out of line and loops are not unrolled (143 KB: 30,000 glyph
 // paths 1.5 times faster). Times, a thread per path and a warp per path: one glyph of 1,083 events
-// 11.6 and 3.0 ms, 777 glyphs 47.8 and 9.9 ms, 30,000 glyphs 361 and 54 ms.
+// 11.6 and 2.9 ms, 777 glyphs 47.8 and 9.8 ms, 30,000 glyphs 361 and 53 ms. Small simple paths of large
+// batches are the thread's (fill.cu has the rule and both sides' figures).
 // Warps per SM, for one glyph / 777 / 30,000: 8 (154 registers) 2.8 / 9.6 / 68 ms, 12 2.9 / 9.6 / 59,
 // 16 (128 registers) 3.0 / 10.0 / 55, 20 3.1 / 10.4 / 53, 24 3.3 / 10.6 / 54, 32 3.8 / 11.3 / 58.
 #pragma once

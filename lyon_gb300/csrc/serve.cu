@@ -10,10 +10,11 @@
 //
 // Stroke requests take microseconds to milliseconds of GPU time, fill requests about ten
 // milliseconds (one path's sweep runs on one warp). With stroke workers configured, the kinds
-// get separate workers: stroke workers run on streams of the device's highest priority with one
-// stroke block per SM, and fill sweeps keep at most `fill_blocks_per_sm` blocks per SM, so that
-// a stroke launch finds room on every SM and starts while fill sweeps are running instead of
-// waiting for them to end.
+// get separate workers: stroke workers run on streams of the device's highest priority, and fill
+// sweeps keep at most `fill_blocks_per_sm` blocks per SM, so that a stroke launch finds room on
+// every SM and starts while fill sweeps are running instead of waiting for them to end. (The
+// kernels that stroke verb by verb are short, and one block's end is another's room; the persistent
+// grid of the paths stroked as a whole is one block per SM.)
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>

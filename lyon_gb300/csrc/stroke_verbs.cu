@@ -24,15 +24,18 @@
 // Emit phase: runs_kernel writes the runs (lane = flattened point), joins_emit_kernel the general
 // joins and the irregular verbs, tails_kernel the tails.
 //
-// A path that breaks the grammar, fails, has a curve of very many steps, or may skip a join goes
-// to a list that stroke.cu walks, one warp per path, with the status that walk gives. Outputs are
+// A path that breaks the grammar, fails, has a curve of very many steps (of few more than its verbs,
+// where one thread would replay them), or may skip a join goes to a list that stroke.cu walks, one
+// warp per path, with the status that walk gives. A batch whose offsets run backwards is stroked by
+// that walk altogether. Outputs are
 // the same bit for bit; tests/test_gpu_stroke_verbs.py compares the two.
 //
 // Measured, whole calls on one GB300, against the warp-per-path walk for every path: 200,000 curve
 // paths (0.47 G vertices) 36.1 -> 8.4 ms, 400,001 map polylines 15.6 -> 1.75 ms, attribute records on
 // 20,000 paths 6.4 -> 2.5 ms (by lyon's stepper, a verb per thread, 4.6), 10,000 curve paths
-// from and to pinned host memory 9.5 -> 3.6 ms, 1,000 paths of 16 segments 287 -> 241 us, one such
-// path from and to host arrays 231 -> 157 us. The walk was bound by the latency of one warp's
+// from and to pinned host memory 9.5 -> 3.6 ms, 1,000 paths of 16 segments 287 -> 250 to 280 us from
+// run to run, one such path from and to host arrays 231 -> 155 us. Many short lines are stroked path by
+// path (api.cu has the rule and both sides' figures). The walk was bound by the latency of one warp's
 // chunks (6,000 to 14,000 cycles for 32 points, its code larger than the instruction cache, the
 // longest path last); here no kernel holds more than one stage's code, and parallelism is in verbs
 // and points.
@@ -1295,8 +1298,8 @@ __global__ void __launch_bounds__(256) paths_kernel(StrokeArgs A, StrokeVerbs S)
 // All that follows the verbs' counts, by one block: with VERBS their positions, then the paths'
 // counts (paths_kernel), the index range per path, the paths' places and the totals (the kernels of
 // scan.cu). For few paths these are short kernels one after another, of which the launches are most:
-// five, with three fills of words before them, for which one path's call took 169 us and takes 157, and
-// 1,000 paths of 16 segments 267 and 241.
+// five, with three fills of words before them, for which one path's call took 169 us and takes 157.
+// (1,000 paths of 16 segments gain less than their spread from run to run.)
 template <bool VERBS>
 __global__ void __launch_bounds__(SCAN_THREADS) finish_kernel(StrokeArgs A, StrokeVerbs S,
                                                               StrokeFinish F) {
