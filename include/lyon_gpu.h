@@ -594,8 +594,9 @@ typedef struct lyon_srv_config {
                                       holding later results can wait forever) */
     uint32_t num_stroke_workers;   /* workers reserved for stroke requests, on streams of the
                                       device's highest priority (the persistent grid of paths
-                                      stroked as a whole: one block per SM), so that their launches start beside running fill sweeps
-                                      instead of queueing behind them; 0 -> none (every worker
+                                      stroked as a whole: one block per SM), so that their
+                                      launches start beside running fill sweeps instead of
+                                      queueing behind them; 0 -> none (every worker
                                       takes both kinds, oldest request first) */
     uint32_t fill_blocks_per_sm;   /* fill sweep blocks per SM for each fill worker; 0 -> 8
                                       with stroke workers (half the library's default), else the

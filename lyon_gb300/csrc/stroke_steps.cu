@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                     }
                     split[lane] = m1;
                     uint32_t incl = (m + 3u) & ~3u;
-    #pragma unroll
+#pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
                         const uint32_t up = __shfl_up_sync(FULL, incl, o);
                         if (lane >= o) incl += up;
@@ -337,9 +337,10 @@ __global__ void __launch_bounds__(256) advance_long_kernel(StrokeArgs A, StrokeV
                         const uint32_t f = first[lane], m1 = split[lane];
                         const float before =
                             (uint32_t)lane == i ? start
-                                                : sum[first[lane - 1] + ((uint32_t)kinds[lane - 1] >> 4) - 1u];
+                                                : sum[first[lane - 1] +
+                                                      ((uint32_t)kinds[lane - 1] >> 4) - 1u];
                         float a[4];
-    #pragma unroll
+#pragma unroll
                         for (uint32_t c = 0; c < 4; ++c)
                             a[c] = m + c >= 4u ? sum[f + m + c - 4u] : m + c == 3u ? before : 0.0f;
                         if (m1) a[0] = sum[f + m1 - 1u];

@@ -467,8 +467,9 @@ __device__ __forceinline__ void store_chain(const StrokeVerbs& S, uint32_t v, ui
 // 3.4 us a verb of the path and, once a batch, 100 us of further launches; in a large batch the other
 // verbs take longer than that one thread. The replay that finds whether the verb can be cut instead
 // takes 0.3 us a step: it is tried for REPLAY_STEPS times as many where points merge at one cusp or
-// none (a drawn cusp; what else there is can hardly be cut). One path of one curve that turns round twice, 1,864 steps: 1266 -> 434 us,
-// by the walk 338; 2,000 paths of ten such curves of 590 steps 3527 -> 1200 us, 976.
+// none (a drawn cusp; what else there is can hardly be cut). One path of one curve that turns round
+// twice, 1,864 steps: 1266 -> 434 us, by the walk 338; 2,000 paths of ten such curves of 590 steps 3527
+// -> 1200 us, by the walk 976.
 __device__ __forceinline__ uint32_t serial_steps(const StrokeArgs& A, uint32_t path, uint32_t nv) {
     const uint32_t verbs = A.verb_offsets[path + 1] - A.verb_offsets[path];
     return max(64u + verbs + verbs / 2u, nv / 500u);
