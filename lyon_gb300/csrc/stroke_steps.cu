@@ -656,8 +656,9 @@ __device__ __forceinline__ void step_verb(const StrokeArgs& A, const StrokeVerbs
         stepper_end<VW>(T, keep, kind == LYON_VERB_CLOSE, P, s, &status, &start_adv);
         // Where the path's next sub-path starts, against what advance_special took: a skipped step
         // replaces a point of a variable-width stroke, and the sum over its points is another one.
-        // (Only records show it.)
-        if (VW && !EMIT && A.vertex_attrs && v + 1u < A.verb_offsets[path + 1] - A.verb_offsets[0] &&
+        // (Not only records show it: a join's fold test takes differences of advancements, which
+        // round by their size.)
+        if (VW && !EMIT && v + 1u < A.verb_offsets[path + 1] - A.verb_offsets[0] &&
             (S.kind[v + 1] & KIND_MASK) == LYON_VERB_BEGIN &&
             !(start_adv == advancement_back(S, v + 1, 0)))
             leave_to_walk(S, path);

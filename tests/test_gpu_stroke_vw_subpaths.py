@@ -102,3 +102,38 @@ def test_rough_paths_of_several_sub_paths(ctx):
         for how in ("widths records", "sources widths records"):
             sv.same_bits(sv.stepped(ctx, batch, o, how, by_path=True),
                          sv.stepped(ctx, batch, o, how))
+
+
+def test_start_that_decides_a_fold(ctx):
+    # A join's fold test takes differences of advancements, which round by their size: with another
+    # start the third sub-path has one vertex more and a triangle less.
+    verbs = [3, 0, 2, 4, 3, 0, 0, 2, 0, 0, 5, 3, 2, 2, 0, 1, 1, 0, 0, 4]
+    pts = [[192.5571, 294.10443], [194.88756, 295.94342], [193.78716, 295.9947],
+           [188.68097, 299.53302], [191.35272, 300.57715], [192.5571, 294.10443],
+           [352.83078, 216.94138], [352.86792, 216.95052], [352.86792, 216.95052],
+           [352.82217, 216.96696], [352.9137, 216.93405], [352.7754, 216.9609],
+           [352.72232, 216.89346], [352.70685, 216.90799], [94.102104, 302.7594],
+           [96.51862, 302.71045], [96.51862, 302.71045], [96.51862, 302.71045],
+           [96.34326, 302.26913], [94.26125, 301.24524], [96.51751, 302.72067],
+           [96.52352, 302.72314], [100.77119, 305.8152], [96.53413, 302.71524],
+           [96.535545, 302.7136], [np.nan, np.nan], [96.544106, 302.72296],
+           [96.53903, 302.7102], [94.102104, 302.7594]]
+    widths = np.array([1.7532835, 1.8890697, 2.0728052, 0.6518197, 1.9705687, 1.525312, 0.84149075,
+                       1.3264579, 2.372185, 1.4872794, 0.84606594, 0.6240128, 1.3036344, 2.102586,
+                       1.0312787, 2.2327008, 1.5148836, 1.6129473, 2.3749108, 1.8366987, 1.8139644,
+                       1.366115, 1.9680815, 2.2341533, 0.88740265, 1.7515548, 0.5827274, 0.7585378,
+                       0.67546785], np.float32)
+    batch = PathBatch(np.array(verbs, np.uint8), np.array(pts, np.float32),
+                      np.array([0, len(verbs)], np.uint32), np.array([0, len(pts)], np.uint32))
+    opts = np.zeros(1, STROKE_OPTIONS_DTYPE)
+    opts["line_width"], opts["miter_limit"], opts["tolerance"] = 0.05, 1.0, 0.003
+    import torch
+    want = orc.batch("stroke", batch, opts, 32, 1, widths=widths)
+    db, od = T.DeviceBatch.upload(batch, 0), T.upload_options(opts, 0)
+    w = torch.from_numpy(widths).cuda()
+    torch.cuda.synchronize()
+    res = T.tessellate_paths("stroke", db, od, 1, 32, T.INDEX_GLOBAL, 0, ctx, widths=w)
+    ctx.synchronize()
+    assert (res.total_vertices, res.total_indices) == (309, 909)
+    assert np.array_equal(res.indices().cpu().numpy().view(np.uint32), want["indices"])
+    assert np.array_equal(res.vertices().cpu().numpy(), want["vertices"], equal_nan=True)
