@@ -102,6 +102,23 @@ def test_small_paths_among_as_many_others(others):
     assert np.array_equal(s["gpu"]["vertices"], s["oracle"]["vertices"])
 
 
+def test_sources_of_small_paths():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import gpu_helpers
+    import test_gpu_fill_custom as custom
+    rng = np.random.default_rng(8)
+    kinds = [_simple(i, rng) for i in range(256)]
+    paths = [kinds[i % 256] for i in range(12400)] + _others(rng)
+    paths = [paths[i] for i in rng.permutation(len(paths))]
+    batch = PathBatch.from_paths(paths)
+    opts = fill_options_array([(0.05, FillRule.NonZero, 0, 1)])
+    attrs = rng.uniform(0, 1, (len(batch.points), 2)).astype(np.float32)
+    bad, _ = custom.compare_fill_custom(gpu_helpers, batch, opts, attrs)
+    assert not bad, bad[:10]
+
+
 def test_time_of_many_simple_paths():
     # 30,000 polygons of 32 points: a thread each takes less time than a warp each would, which is
     # what the same batch takes in three calls of 10,000.
